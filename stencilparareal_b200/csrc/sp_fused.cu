@@ -43,6 +43,7 @@
 #include <type_traits>
 #include <utility>
 
+#include "sp_column.cuh"
 #include "sp_device.cuh"
 #include "sp_internal.h"
 #include "sp_stencil.cuh"
@@ -468,21 +469,23 @@ __global__ void __launch_bounds__(TY * TXP / 2, TY * TXP / 2 <= 256 ? 2 : 1)
 // ---------------------------------------------------------------------------
 // Widening: interior of a caller-layout field -> internal field with every
 // periodic image within 4 cells of a face.
-__global__ void k_widen(double* dst, Geo gd, const double* src, Geo gs, int items, const int* item_lo,
-                        int item_base, StoreBounds bounds) {
+__global__ void __launch_bounds__(kColX * kColY)
+    k_widen(double* dst, Geo gd, const double* src, Geo gs, int items, const int* item_lo, int item_base,
+            StoreBounds bounds) {
     pdl_trigger();
     pdl_wait();
-    const long long n = (long long)gd.ni * gd.nj * gd.nk;
-    const int b = blockIdx.y;
+    const int b = blockIdx.z;
     if (item_lo && b + item_base < *item_lo) return;
-    const double* sb = src + (long long)b * gs.total + gs.origin;
+    const double* sb = src + (long long)b * gs.total;
     double* db = dst + (long long)b * gd.total + gd.origin;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(t % gd.ni);
-        const int y = (int)((t / gd.ni) % gd.nj);
-        const int z = (int)(t / ((long long)gd.ni * gd.nj));
-        const double v = sb[(long long)z * gs.plane + (long long)y * gs.px + x];
-        const int hd = gd.halo;
+    const int hd = gd.halo;
+    for_column(gd, [&](int x, int y, int z) {
+        const double v = sb[cell_at(gs, x, y, z)];
+        const bool inner = x >= hd && x < gd.ni - hd && y >= hd && y < gd.nj - hd && z >= hd && z < gd.nk - hd;
+        if (inner) {
+            gst1(bounds, db + z * gd.plane + y * gd.px + x, v);
+            return;
+        }
 #pragma unroll
         for (int iz = 0; iz < 3; ++iz) {
             if (iz == 1 && !(z < hd)) continue;
@@ -499,7 +502,7 @@ __global__ void k_widen(double* dst, Geo gd, const double* src, Geo gs, int item
                 if (x >= gd.ni - hd) gst1(bounds, r + x - gd.ni, v);
             }
         }
-    }
+    });
 }
 
 template <int PAIR, int TY, int NSQ, int NP, int TXP>
@@ -568,11 +571,6 @@ cudaError_t set_pair_attr() {
                                 (int)PairShape<TY, NSQ, NP, PAIR, TXP>::smem);
 }
 
-unsigned grid_cells(long long n) {
-    const long long b = (n + 255) / 256;
-    return (unsigned)(b < 148 * 16 ? b : 148 * 16);
-}
-
 }  // namespace
 
 bool pair_supported(const Geo& g) { return g.es == 8 && g.ni >= 4 && g.nj >= 4 && g.nk >= 4; }
@@ -618,8 +616,7 @@ cudaError_t launch_widen(const Geo& g4, void* dst, const Geo& gs, const void* sr
                          int item_base, cudaStream_t s) {
     add_launches(1);
     if (g4.es != 8 || gs.es != 8 || items < 1 || items > 65535) return cudaErrorInvalidValue;
-    dim3 grid(grid_cells((long long)g4.ni * g4.nj * g4.nk), items);
-    return launch_pdl(k_widen, grid, dim3(256), 0, s, static_cast<double*>(dst), g4,
+    return launch_pdl(k_widen, column_grid(g4, items, 4), dim3(kColX, kColY), 0, s, static_cast<double*>(dst), g4,
                       static_cast<const double*>(src), gs, items, item_lo, item_base, out_bounds(dst, g4, items));
 }
 

@@ -178,9 +178,6 @@ cudaError_t launch_zero_item(void* base, long long bytes, int nitems, const int*
                              int min_item = 0);
 // err[0] += sum (a-b)^2 ; err[1] += sum b^2 ; err[2] = max |a-b| ; err[3] = max |a|   (FP64 fields)
 cudaError_t launch_errors(const Geo& g, const double* a, const double* b, double* acc4, cudaStream_t s);
-// Pointwise axpby on FP64 fields (interior+images): out = alpha*x + beta*y (y may be null).
-cudaError_t launch_axpby(const Geo& g, double* out, double alpha, const double* x, double beta, const double* y,
-                         cudaStream_t s);
 // 0.5*||a-b||^2 and lam = a - b (lam may alias nothing; written with images).
 cudaError_t launch_misfit(const Geo& g, const double* a, const double* b, double* lam, double* jacc, cudaStream_t s);
 
