@@ -593,6 +593,29 @@ cudaError_t prepare_pairs() {
     return e;
 }
 
+// Tiles of 32 x 16 cells with as many z-ranges as fill two waves of CTAs (two per
+// SM), no range longer than 64 planes -- or 64 x 8 over one range per resident CTA
+// where those pad the plane less.  us per step, 32 x 16 / 64 x 8: 192^3 (24 planes)
+// 155 / 158, 256^3 (64 planes) 315 / 325, 8 fields of 96^3 161 / 212; 8 of 100^3
+// (128 x 112 against 128 x 104 cells) 244 / 235.
+Shape default_pair_shape(const Geo& g, int items) {
+    auto padded = [&](int tx, int ty) {
+        return (long long)((g.ni + tx - 1) / tx) * tx * ((g.nj + ty - 1) / ty) * ty;
+    };
+    Shape sh;
+    if (padded(64, 8) < padded(32, 16)) {
+        sh.ty = 8;
+        sh.zchunk = 0;
+        return sh;
+    }
+    const long long tiles = padded(32, 16) / 512 * items;
+    const long long ranges = std::max((g.nk + 63) / 64LL, std::max(1LL, 4 * 148 / tiles));
+    sh.tx = 32;
+    sh.ty = 16;
+    sh.zchunk = (int)std::max(1LL, (g.nk + ranges - 1) / ranges);
+    return sh;
+}
+
 cudaError_t launch_pair(const Geo& g4, const Geo& go, const PairLaunch& L, const Shape& sh, cudaStream_t s,
                         int* err) {
     add_launches(1);

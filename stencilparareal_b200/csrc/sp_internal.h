@@ -46,7 +46,9 @@ constexpr int kNumOps = OP_ADJ + 4;
 struct Tune {
     Shape op[kNumOps];
     Shape pair[2] = {Shape{8, 0, 1}, Shape{8, 0, 1}};  // fused stage pairs 1+2 and 3+4 (ty 8 or 16)
-    int fused = 0;    // 1: FP64 RK4 steps run as the two fused pairs
+    int fused = 0;    // 1: FP64 RK4 steps run as the two fused pairs ...
+    int direct = 0;   // ... 1: except that launches this small run on the stage kernels of `op`
+    bool pairs() const { return fused && !direct; }
     int cluster = 0;  // FP64 RK4 propagations of small fields run cluster-resident (sp_cluster.cu):
                       // 1 on z-slabs, 2 on (y,z) blocks
     void set_all(const Shape& s) {
@@ -121,6 +123,9 @@ size_t cluster_weights_bytes();
 void fill_cluster_weights(void* w13, const Coef& c, double nu);  // one entry of wtab (host memory)
 constexpr int kClusterSmemMax = 227 * 1024;
 
+// Launch shape of the single-stage kernels before tuning, for `items` fields per launch.
+Shape default_stage_shape(const Geo& g, int items, bool adjoint = false);
+
 // Launches one stage kernel; counts the launch.  err: device error word.
 cudaError_t launch_stage(const Geo& g, const StageLaunch& L, const Tune& t, cudaStream_t s, int* err);
 
@@ -142,6 +147,7 @@ struct PairLaunch {
     Coef coef;
 };
 bool pair_supported(const Geo& g);  // FP64, at least 4 interior cells per dimension
+Shape default_pair_shape(const Geo& g, int items);  // before tuning
 cudaError_t launch_pair(const Geo& g4, const Geo& go, const PairLaunch& L, const Shape& sh, cudaStream_t s, int* err);
 // dst (geometry g4) <- interior of src (geometry gs), with g4.halo-deep images (FP64, items fields).
 cudaError_t launch_widen(const Geo& g4, void* dst, const Geo& gs, const void* src, int items, const int* item_lo,

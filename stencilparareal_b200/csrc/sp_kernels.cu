@@ -18,9 +18,9 @@
 // plus nu * Laplace4 (ConvectionFunctions.h:135-167), written as
 //   R = sum_d c_d/(12dx) * (8(q[-1]-q[+1]) - (q[-2]-q[+2]))_d
 //     + nu/(12dx^2) * (16 S1 - S2 - 90 q),  S1/S2 = sums of the +-1/+-2 neighbours,
-// the same coefficients regrouped into differences (the direct-load kernel and
-// the adjoint); the TMA RK stages use them combined into 13 per-offset weights
-// (rhs_w13, sp_stencil.cuh), as the fused stage pairs do.  R2 is RHS2Stage
+// the same coefficients regrouped into differences (the adjoint, and RK stages
+// with one diffusivity per item); the other RK stages use them combined into 13
+// per-offset weights (rhs_w13, sp_stencil.cuh), as the fused stage pairs do.  R2 is RHS2Stage
 // (Convection.cpp:30-55) with the upwind Advection2 (ConvectionFunctions.h:18-42).
 //
 // Fields carry a 2-cell halo (layout in include/sp_abi.h).  Every kernel that
@@ -34,12 +34,13 @@
 //    shared-memory slots completed on mbarriers; pointwise operands arrive the
 //    same way.  The z-neighbours live in registers.  16-byte shared and global
 //    accesses, VX = 2 (FP64) or 4 (FP32) cells per thread.
-//  * k_stage_direct: one thread per column, loads straight from global memory
-//    through L1; used for cross-checking and when the tuner prefers it.
+//  * k_stage_direct: one 16-byte chunk of a row per thread, loads straight from
+//    global memory through L1: the faster one for small launches.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <mutex>
@@ -140,6 +141,23 @@ __device__ __forceinline__ T diff_mode(int m, T c, T lo, T hi) {
     return m == 0 ? c - lo : (m == 1 ? hi - c : lo - hi);
 }
 
+// The RK update of one cell from k = R(stencil input): c the stencil input's
+// centre, q0, q1 the pointwise operands.
+template <typename T, int OP>
+__device__ __forceinline__ void rk_update(const KArgs<T>& a, T k, T c, T q0, T q1, T& oy, T& oa) {
+    if constexpr (OP == OP_RK_S1) {
+        oy = fmaT(a.c_y, k, c);
+    } else if constexpr (OP == OP_RK_S2) {
+        oy = fmaT(a.c_y, k, q0);
+        oa = fmaT(a.c_acc, k, add_third(c, q0, q0));
+    } else if constexpr (OP == OP_RK_S3) {
+        oy = fmaT(a.c_y, k, q0);
+    } else {
+        oy = fmaT(a.c_acc, k, add_third(c, q1, q0));
+    }
+    (void)q0; (void)q1; (void)oa;
+}
+
 // One cell of one stage.  p0..p2: pointwise operands; oy/oa: outputs;
 // g[4]: adjoint parameter partial sums (unscaled).
 template <typename T, int OP>
@@ -182,17 +200,8 @@ __device__ __forceinline__ void cell_op(const KArgs<T>& a, T nl, const Nb<T>& s,
         const T adv = fmaT(a.ca0, ax, fmaT(a.ca1, ay, a.ca2 * az));
         if constexpr (!OpTraits<OP>::adjoint) {
             const T k = fmaT(nl, lap, adv);
-            if constexpr (OP == OP_RK_S1) {
-                oy = fmaT(a.c_y, k, s.c);
-            } else if constexpr (OP == OP_RK_S2) {
-                oy = fmaT(a.c_y, k, p0);
-                oa = fmaT(a.c_acc, k, add_third(s.c, p0, p0));
-            } else if constexpr (OP == OP_RK_S3) {
-                oy = fmaT(a.c_y, k, p0);
-            } else {  // S4
-                oy = fmaT(a.c_acc, k, add_third(s.c, p1, p0));
-            }
-            (void)g; (void)live; (void)p1; (void)oa;
+            rk_update<T, OP>(a, k, s.c, p0, p1, oy, oa);
+            (void)g; (void)live;
         } else {
             // R^T m = -sum_d c_d D_d m + nu L m (D_d antisymmetric, L symmetric on the periodic grid)
             const T ybar = a.sigma * fmaT(nl, lap, -adv);
@@ -215,20 +224,6 @@ __device__ __forceinline__ void cell_op(const KArgs<T>& a, T nl, const Nb<T>& s,
     }
 }
 
-// Stores one value and its periodic images.  base = interior origin of the item.
-template <typename T>
-__device__ __forceinline__ void store_images1(T* base, int x, int y, int z, T v, const KArgs<T>& a) {
-    T* row = base + (long long)z * a.plane + (long long)y * a.px;
-    const StoreBounds& b = a.sb_y;
-    gst1(b, row + x, v);
-    if (x < 2) gst1(b, row + x + a.ni, v);
-    if (x >= a.ni - 2) gst1(b, row + x - a.ni, v);
-    if (y < 2) gst1(b, row + (long long)a.nj * a.px + x, v);
-    if (y >= a.nj - 2) gst1(b, row - (long long)a.nj * a.px + x, v);
-    if (z < 2) gst1(b, row + (long long)a.nk * a.plane + x, v);
-    if (z >= a.nk - 2) gst1(b, row - (long long)a.nk * a.plane + x, v);
-}
-
 template <typename T, int N>
 __device__ __forceinline__ void put_vec(const StoreBounds& b, T* p, int x, int ni, const Vec<T, N>& v) {
     if (x + N <= ni) {
@@ -242,12 +237,11 @@ __device__ __forceinline__ void put_vec(const StoreBounds& b, T* p, int x, int n
 
 // Vector store of cells x..x+N-1 of row (y,z) plus periodic images.
 template <typename T, int N>
-__device__ __forceinline__ void store_images_vec(T* base, int x, int y, int z, const Vec<T, N>& v, const KArgs<T>& a,
-                                                 bool images) {
+__device__ __forceinline__ void store_images_vec(T* base, int x, int y, int z, const Vec<T, N>& v,
+                                                 const KArgs<T>& a) {
     T* row = base + (long long)z * a.plane + (long long)y * a.px + x;
     const StoreBounds& b = a.sb_y;
     put_vec<T, N>(b, row, x, a.ni, v);
-    if (!images) return;
 #pragma unroll
     for (int e = 0; e < N; ++e) {
         const int xe = x + e;
@@ -290,46 +284,108 @@ __device__ __forceinline__ void reduce_par(double* g, double* par_acc, double gs
 }
 
 // ---------------------------------------------------------------------------
-// Direct-load stage kernel: block (32, TYD), one thread per (x, y) column,
-// marching zchunk planes; grid (ceil(ni/32), ceil(nj/TYD), nzc * items).
-template <typename T, int OP, int TYD>
-__global__ void __launch_bounds__(32 * TYD) k_stage_direct(const KArgs<T> a) {
-    const int zc = blockIdx.z % a.nzc;
-    const int b = blockIdx.z / a.nzc;
+// Direct-load stage kernel: a thread owns one 16-byte chunk (2 FP64 or 4 FP32
+// cells) of one row and marches zchunk planes, everything loaded straight from
+// global memory (L1 serves the reuse between the block's rows).  The chunks of a
+// plane are numbered row by row, so that a row of any width fills its warps;
+// grid (ceil(chunks / threads), nzc, items).
+//
+// Bound by latency at the sizes it is for: below ~4M FP64 cells a stage is one
+// short wave, and what counts is the time from launch to the last store.  Hence
+// no barrier and no shared-memory ring to fill, few registers (50-64 for the
+// FP64 RK stages: 16 or more blocks of 128 threads per SM), a compact plane loop
+// (not unrolled: 2-3 KB of code per stage instead of 10-25 KB, which the short
+// kernels spent their time fetching) and programmatic dependent launch.  us per
+// RK4 step, one-thread-per-cell direct kernel / best TMA ring / this kernel:
+//   FP64  64^3 16.2 / 25.6 / 12.6   96^3 29.5 / 34.5 / 23.5   128^3 57.4 / 53.2 / 51.2   192^3 196 / 156 / 175
+//   FP32  64^3 17.7 / 27.2 / 13.3   96^3 30.6 / 30.8 / 18.9   128^3 56.4 / 34.9 / 32.2   192^3 167 / 112 / 102
+// Unrolled by two with the next plane prefetched (70-100 registers): 64^3 FP32
+// 11.0, but 128^3 FP64 62.5 and FP32 41.8.
+
+// A chunk by a plain global load.  Not volatile, so that the compiler may move it
+// over the stores of other cells; the addresses come from pointers passed
+// through after_wait, so that it cannot move over griddepcontrol.wait.
+template <typename T>
+__device__ __forceinline__ Vec<T, V16<T>::N> ldg16(const T* p) {
+    Vec<T, V16<T>::N> r;
+    if constexpr (sizeof(T) == 8)
+        asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.v[0]), "=d"(r.v[1]) : "l"(p));
+    else
+        asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]) : "l"(p));
+    return r;
+}
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+
+template <typename T, int OP, bool PER_ITEM>
+__global__ void __launch_bounds__(512) k_stage_direct(const __grid_constant__ KArgs<T> a) {
+    constexpr int N = V16<T>::N, NPW = OpTraits<OP>::npw;
+    constexpr bool RK = OP <= OP_RK_S4;
+    using V = Vec<T, N>;
+    pdl_trigger();
+    pdl_wait();
+    const int b = blockIdx.z;
     if (a.item_lo && b + a.item_base < *a.item_lo) return;
-    const int x = blockIdx.x * 32 + threadIdx.x;
-    const int y = blockIdx.y * TYD + threadIdx.y;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = t / a.tiles_x;  // tiles_x: chunks per row
+    const int x = (t - y * a.tiles_x) * N;
     double g[4] = {0., 0., 0., 0.};
-    const bool live = x < a.ni && y < a.nj;
-    if (live) {
+    if (y < a.nj) {
+        const int z0 = (a.zrev ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y) * a.zchunk;
+        const int z1 = min(z0 + a.zchunk, a.nk);
         const long long ob = (long long)b * a.item_stride + a.origin;
         const long long col = ob + (long long)y * a.px + x;
-        const T* S = a.yin + col;
-        const int z0 = zc * a.zchunk;
-        const int z1 = min(z0 + a.zchunk, a.nk);
+        const T* S = after_wait(a.yin) + col;
+        [[maybe_unused]] const T* pw[3] = {nullptr, nullptr, nullptr};
+        if constexpr (NPW > 0) pw[0] = after_wait(a.pw0) + col;
+        if constexpr (NPW > 1) pw[1] = after_wait(a.pw1) + col;
+        if constexpr (NPW > 2) pw[2] = after_wait(a.pw2) + col;
         const T nl = item_nl(a, b);
-        const long long pl = a.plane;
-        T zm2 = __ldg(S + (z0 - 2) * pl), zm1 = __ldg(S + (z0 - 1) * pl);
-        T zc0 = __ldg(S + z0 * pl), zp1 = __ldg(S + (z0 + 1) * pl);
+        const long long pl = a.plane, px = a.px;
+        V win[5];  // the column's planes z-2 .. z+2
+#pragma unroll
+        for (int i = 0; i < 4; ++i) win[i] = ldg16<T>(S + (z0 - 2 + i) * pl);
+#pragma unroll 1
         for (int z = z0; z < z1; ++z) {
-            const T zp2 = __ldg(S + (z + 2) * pl);
-            const T* P = S + z * pl;
-            Nb<T> s;
-            s.c = zc0; s.zm1 = zm1; s.zp1 = zp1; s.zm2 = zm2; s.zp2 = zp2;
-            s.xm1 = __ldg(P - 1); s.xp1 = __ldg(P + 1); s.xm2 = __ldg(P - 2); s.xp2 = __ldg(P + 2);
-            s.ym1 = __ldg(P - a.px); s.yp1 = __ldg(P + a.px);
-            s.ym2 = __ldg(P - 2 * a.px); s.yp2 = __ldg(P + 2 * a.px);
-            const long long off = col + z * pl;
-            T p0 = 0, p1 = 0, p2 = 0;
-            constexpr int NPW = OpTraits<OP>::npw;
-            if constexpr (NPW > 0) p0 = a.pw0[off];
-            if constexpr (NPW > 1) p1 = a.pw1[off];
-            if constexpr (NPW > 2) p2 = a.pw2[off];
-            T oy = 0, oa = 0;
-            cell_op<T, OP>(a, nl, s, p0, p1, p2, oy, oa, g, true);
-            store_images1<T>(a.yout + ob, x, y, z, oy, a);
-            if constexpr (OpTraits<OP>::writes_a) gst1(a.sb_a, a.aout + off, oa);
-            zm2 = zm1; zm1 = zc0; zc0 = zp1; zp1 = zp2;
+            const long long zo = z * pl;
+            const T* P = S + zo;
+            win[4] = ldg16<T>(P + 2 * pl);
+            const V xl = ldg16<T>(P - N), xr = ldg16<T>(P + N);
+            const V ym1 = ldg16<T>(P - px), yp1 = ldg16<T>(P + px);
+            const V ym2 = ldg16<T>(P - 2 * px), yp2 = ldg16<T>(P + 2 * px);
+            [[maybe_unused]] V p[3];
+#pragma unroll
+            for (int k = 0; k < NPW; ++k) p[k] = ldg16<T>(pw[k] + zo);
+            T row[3 * N];
+#pragma unroll
+            for (int e = 0; e < N; ++e) { row[e] = xl.v[e]; row[N + e] = win[2].v[e]; row[2 * N + e] = xr.v[e]; }
+            V oy, oa;
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                Nb<T> s;
+                s.c = row[N + e];
+                s.xm1 = row[N + e - 1]; s.xp1 = row[N + e + 1];
+                s.xm2 = row[N + e - 2]; s.xp2 = row[N + e + 2];
+                s.ym1 = ym1.v[e]; s.yp1 = yp1.v[e]; s.ym2 = ym2.v[e]; s.yp2 = yp2.v[e];
+                s.zm1 = win[1].v[e]; s.zp1 = win[3].v[e]; s.zm2 = win[0].v[e]; s.zp2 = win[4].v[e];
+                T q0 = 0, q1 = 0, q2 = 0, vy = 0, va = 0;
+                if constexpr (NPW > 0) q0 = p[0].v[e];
+                if constexpr (NPW > 1) q1 = p[1].v[e];
+                if constexpr (NPW > 2) q2 = p[2].v[e];
+                if constexpr (RK && !PER_ITEM) rk_update<T, OP>(a, rhs_w13(a.w, s), s.c, q0, q1, vy, va);
+                else cell_op<T, OP>(a, nl, s, q0, q1, q2, vy, va, g, x + e < a.ni);
+                oy.v[e] = vy;
+                oa.v[e] = va;
+            }
+            const bool edge = x < 2 || x + N > a.ni - 2 || y < 2 || y >= a.nj - 2 || z < 2 || z >= a.nk - 2;
+            if (!edge) gst16<T>(a.sb_y, a.yout + col + zo, oy);
+            else store_images_vec<T, N>(a.yout + ob, x, y, z, oy, a);
+            if constexpr (OpTraits<OP>::writes_a) put_vec<T, N>(a.sb_a, a.aout + col + zo, x, a.ni, oa);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) win[i] = win[i + 1];
         }
     }
     if constexpr (OpTraits<OP>::adjoint) reduce_par(g, a.par_acc, a.gs_nu, a.gs_c);
@@ -523,17 +579,7 @@ __global__ void __launch_bounds__(32 * TY)
             if constexpr (NPA > 2) q2 = p2v.v[e];
             T vy = 0, va = 0;
             if constexpr (RK) {
-                const T k = rhs_w13(a.w, s);
-                if constexpr (OP == OP_RK_S1) {
-                    vy = fmaT(a.c_y, k, s.c);
-                } else if constexpr (OP == OP_RK_S2) {
-                    vy = fmaT(a.c_y, k, q0);
-                    va = fmaT(a.c_acc, k, add_third(s.c, q0, q0));
-                } else if constexpr (OP == OP_RK_S3) {
-                    vy = fmaT(a.c_y, k, q0);
-                } else {
-                    vy = fmaT(a.c_acc, k, add_third(s.c, q1, q0));
-                }
+                rk_update<T, OP>(a, rhs_w13(a.w, s), s.c, q0, q1, vy, va);
             } else {
                 cell_op<T, OP>(a, nl, s, q0, q1, q2, vy, va, g, live && x + e < a.ni);
             }
@@ -551,7 +597,7 @@ __global__ void __launch_bounds__(32 * TY)
                     }
                 }
             } else {
-                store_images_vec<T, VX>(a.yout + ob, x, y, z, oy, a, true);
+                store_images_vec<T, VX>(a.yout + ob, x, y, z, oy, a);
             }
             if constexpr (OpTraits<OP>::writes_a) {
                 if (full_vec) gst16<T>(a.sb_a, arow_out, oa);
@@ -670,17 +716,16 @@ KArgs<T> make_args(const Geo& g, const StageLaunch& L, const Shape& t, int* err)
 }
 
 template <typename T, int OP>
-cudaError_t launch_direct_T(const Geo& g, const KArgs<T>& a, const Shape& t, int items, cudaStream_t s) {
-    const int tyd = t.ty;
-    dim3 grid((g.ni + 31) / 32, (g.nj + tyd - 1) / tyd, a.nzc * items);
-    if (grid.z > 65535u) return cudaErrorInvalidConfiguration;
-    switch (tyd) {
-        case 4: k_stage_direct<T, OP, 4><<<grid, dim3(32, 4), 0, s>>>(a); break;
-        case 8: k_stage_direct<T, OP, 8><<<grid, dim3(32, 8), 0, s>>>(a); break;
-        case 16: k_stage_direct<T, OP, 16><<<grid, dim3(32, 16), 0, s>>>(a); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+cudaError_t launch_direct_T(const Geo& g, KArgs<T> a, const Shape& t, int items, cudaStream_t s) {
+    if (t.ty != 4 && t.ty != 8 && t.ty != 16) return cudaErrorInvalidValue;
+    const unsigned threads = 32u * (unsigned)t.ty;
+    a.tiles_x = (g.ni + V16<T>::N - 1) / V16<T>::N;
+    const long long chunks = (long long)a.tiles_x * g.nj;
+    const dim3 grid((unsigned)((chunks + threads - 1) / threads), (unsigned)a.nzc, (unsigned)items);
+    if (chunks > 0x7fffffffLL || grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
+    if constexpr (OP <= OP_RK_S4)
+        if (a.nu_items) return launch_pdl(k_stage_direct<T, OP, true>, grid, dim3(threads), 0, s, a);
+    return launch_pdl(k_stage_direct<T, OP, false>, grid, dim3(threads), 0, s, a);
 }
 
 template <typename T, int OP, int TY, int NS, int NP>
@@ -735,10 +780,13 @@ cudaError_t launch_tma_op(const Geo& g, const StageLaunch& L, const KArgs<T>& a,
 }
 
 template <typename T>
-cudaError_t launch_T(const Geo& g, const StageLaunch& L, const Shape& t, cudaStream_t s, int* err) {
-    KArgs<T> a = make_args<T>(g, L, t, err);
-    // one diffusivity per item (batched slices with nufreq != 0): direct kernel
+cudaError_t launch_T(const Geo& g, const StageLaunch& L, Shape t, cudaStream_t s, int* err) {
+    // one diffusivity per item (batched slices with nufreq != 0): direct kernel, on
+    // its own shape where the given one is the TMA ring's (16 fields of 64^3: 149
+    // us per step against 161 on 4 rows x 8 planes)
     const bool tma = t.tma && !L.nu_items;
+    if (t.tma && !tma) t = Shape{8, 4, 0};
+    KArgs<T> a = make_args<T>(g, L, t, err);
 #define SP_OPCASE(OPV)                                                              \
     case OPV:                                                                       \
         return tma ? launch_tma_op<T, OPV>(g, L, a, t, s)                           \
@@ -810,6 +858,36 @@ cudaError_t launch_wait_selftest(int* err, unsigned long long limit_ns, cudaStre
     add_launches(1);
     k_wait_selftest<<<1, 64, 0, s>>>(err, limit_ns);
     return cudaGetLastError();
+}
+
+// The direct kernel up to a number of cells per launch, the TMA rings beyond.
+// Where the lines lie (us per RK4 step, direct / TMA): FP64 8 fields of 64^3 (2.1M
+// cells) 58 / 60, 16 of them 126 / 114, one 192^3 175 / 159; FP32 192^3 (7.1M) 102 /
+// 112, 256^3 234 / 204; adjoint (a whole gradient, per step) 96^3 110 / 129, 128^3
+// 251 / 197 -- its direct kernels need 98 registers.  The direct kernel takes as
+// many planes per thread as give one wave of threads (FP64 96^3: 3 planes 23.5, 1
+// or 2 planes 26-27; FP32 95 x 97 x 93: 1 plane 19.9, 2 planes 22.4), at most four
+// (longer chunks gained nothing at 128^3-192^3).
+Shape default_stage_shape(const Geo& g, int items, bool adjoint) {
+    const long long direct = adjoint ? 1'500'000 : (g.es == 8 ? 3'000'000 : 12'000'000);
+    const long long cells = (long long)g.ni * g.nj * g.nk * items;
+    const int n = 16 / g.es;
+    Shape sh;
+    if (cells <= direct) {
+        const long long threads = (long long)((g.ni + n - 1) / n) * g.nj * g.nk * items;
+        const long long wave = 148LL * (g.es == 8 ? 1024 : 1792);
+        sh.tma = 0;
+        sh.ty = g.es == 8 ? 8 : 4;
+        sh.zchunk = (int)std::min(4LL, (threads + wave - 1) / wave);
+        return sh;
+    }
+    // TMA rings: 4-row tiles, z-chunks that give at least ~8 CTAs per SM
+    sh.ty = 4;
+    const long long tiles = (long long)((g.ni + 32 * n - 1) / (32 * n)) * ((g.nj + 3) / 4) * items;
+    int zc = g.nk;
+    while (zc > 8 && tiles * ((g.nk + zc - 1) / zc) < 148LL * 8) zc = (zc + 1) / 2;
+    sh.zchunk = zc;
+    return sh;
 }
 
 cudaError_t launch_stage(const Geo& g, const StageLaunch& L, const Tune& t, cudaStream_t s, int* err) {

@@ -134,24 +134,15 @@ struct sp_convection {
     Tune tune(int prec, int items) {
         auto it = tunes.find({prec, items});
         if (it != tunes.end()) return it->second;
-        // default before tuning: TMA pipeline, 4-row tiles, z-chunks that give
-        // at least ~8 CTAs per SM, the same shape for every stage
-        Shape sh;
-        sh.ty = 4;
-        const int VX = prec == 0 ? 2 : 4;
-        const long long tiles = (long long)((P.ni + 32 * VX - 1) / (32 * VX)) * ((P.nj + 3) / 4) * items;
-        int zc = P.nk;
-        while (zc > 8 && tiles * ((P.nk + zc - 1) / zc) < 148LL * 8) zc = (zc + 1) / 2;
-        sh.zchunk = std::max(1, zc);
+        const Shape sh = default_stage_shape(g[prec], items);
         Tune t;
         t.set_all(sh);
-        // FP64 RK4: fused stage pairs, 8-row tiles, one plane range per resident CTA
+        for (int i = 0; i < 4; ++i) t.op[OP_ADJ + i] = default_stage_shape(g[prec], items, true);
+        // FP64 RK4: fused stage pairs, except in the direct kernel's sizes
         if (prec == 0 && pair_supported(g4)) {
-            Shape ps;
-            ps.ty = 8;
-            ps.zchunk = 0;
-            t.pair[0] = t.pair[1] = ps;
+            t.pair[0] = t.pair[1] = sh.tma ? default_pair_shape(g4, items) : Shape{8, 0, 1};
             t.fused = 1;
+            t.direct = sh.tma ? 0 : 1;
         }
         return t;
     }
@@ -421,7 +412,7 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
         }
         SP_CUDA(launch_rk4_cluster(g, L, s, err));
         SP_CUDA(launch_periodicity(g, out, 1, s));
-    } else if (rk && t.fused && prec == 0 && pair_supported(h->g4)) {
+    } else if (rk && t.pairs() && prec == 0 && pair_supported(h->g4)) {
         // fused stage pairs: widen the input once, alternate the step-start
         // field between wbuf(0) and wbuf(1), write the last step to `out`
         if ((rc = h->ensure_wide(1))) return rc;
@@ -598,6 +589,7 @@ int sp_set_tune(sp_convection* h, int precision, int batch, int ty, int zchunk, 
         sh.tx = kind == 4 ? 32 : 64;
         t.pair[0] = t.pair[1] = sh;
         t.fused = 1;
+        t.direct = 0;
         h->tunes[{precision, batch}] = t;
         h->drop_graphs();
         return SP_OK;
@@ -903,7 +895,7 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
     SP_CUDA(cudaEventCreate(&e0));
     SP_CUDA(cudaEventCreate(&e1));
     Tune best = h->tune(precision, batch);
-    std::vector<int> zcs = {4, 8, 16, 32, 64};
+    std::vector<int> zcs = {1, 2, 3, 4, 8, 16, 32, 64};
     zcs.push_back(g.nk);
     float op_ms[kNumOps];
     for (auto& m : op_ms) m = 1e30f;
@@ -920,7 +912,7 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
         for (int kind = 1; kind >= 0; --kind)
             for (int ty : {4, 8, 16})
                 for (int zc : zcs) {
-                    if (zc > g.nk && zc != g.nk) continue;
+                    if (zc > g.nk || (kind && zc < 4 && zc != g.nk)) continue;
                     if ((long long)((g.nk + zc - 1) / zc) > 65535) continue;
                     Tune t;
                     Shape sh;
@@ -944,7 +936,7 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
     }
     // fused stage pairs (FP64): best shape per pair, then fused or single-stage
     // steps by timing whole steps of both paths
-    best.fused = 0;
+    best.fused = best.direct = 0;
     if (precision == SP_F64 && pair_supported(h->g4)) {
         const Geo& g4 = h->g4;
         const size_t wb = (size_t)batch * g4.total * g4.es;
@@ -1368,7 +1360,7 @@ bool cluster_sweep(const sp_parareal* pr) {
 }
 bool fused_sweep(const sp_parareal* pr) {
     sp_convection* h = pr->prop;
-    return !cluster_sweep(pr) && h->P.nufreq == 0. && h->tune(0, pr->P).fused && pair_supported(h->g4);
+    return !cluster_sweep(pr) && h->P.nufreq == 0. && h->tune(0, pr->P).pairs() && pair_supported(h->g4);
 }
 
 // Allocates the fine-sweep scratch of the path the tune selects; must run

@@ -1,0 +1,93 @@
+"""GPU tests of the direct-load stage kernel and of the default choice between it,
+the TMA rings and the fused pairs.
+
+All of them evaluate the RK4 stages (and Euler) with the same operations in the
+same order, so the fields must agree bit for bit; with one diffusivity per slice
+the direct kernel sums in another order and is held to the oracle.
+"""
+import numpy as np
+import pytest
+
+from ics import gaussian_noise, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# widths around the 16-byte chunk (2 FP64, 4 FP32 cells), rows around a block's warps
+GRIDS = [(32, 32, 32), (17, 19, 23), (2, 3, 5), (5, 4, 2), (130, 66, 7), (4, 130, 9)]
+
+
+def conv_of(sp, n, **kw):
+    a = dict(nu0=0.02, nufreq=0.0, cx=1.0, cy=-0.5, cz=0.25, upwind=True)
+    a.update(kw)
+    return sp.Convection(*n, 1.0 / n[0], a["nu0"], a["nufreq"], a["cx"], a["cy"], a["cz"], upwind=a["upwind"])
+
+
+def steps(sp, c, prec, q0, tune, euler=False, n=3):
+    c.set_tune(prec, 1, *tune)
+    a, b = c.field(prec), c.field(prec)
+    c.upload(a, q0)
+    (c.DoEuler if euler else c.DoRK4)(a, b, 0.0, 1e-4, n)
+    return c.download(b), b
+
+
+def halo_ok(c, f):
+    """The face halos of f are what Periodicity makes of its interior."""
+    before = f.data.clone()
+    c.Periodicity(f)
+    c.synchronize()
+    lay, (ni, nj, nk) = f.layout, (f.ni, f.nj, f.nk)
+    for k, j in [(k, j) for k in range(-2, nk + 2) for j in range(-2, nj + 2)]:
+        if (0 <= k < nk) + (0 <= j < nj) < 1:
+            continue
+        inside = 0 <= k < nk and 0 <= j < nj
+        o = lay.origin + k * lay.plane + j * lay.px
+        lo, hi = (o - 2, o + ni + 2) if inside else (o, o + ni)
+        if not bool((before[lo:hi] == f.data[lo:hi]).all()):
+            return False
+    return True
+
+
+@pytest.mark.parametrize("n", GRIDS)
+@pytest.mark.parametrize("prec", [0, 1], ids=["f64", "f32"])
+def test_direct_equals_tma(sp, n, prec):
+    c = conv_of(sp, n)
+    q0 = gaussian_noise(*n, seed=5)
+    want, _ = steps(sp, c, prec, q0, (4, 8, 1))
+    for tune in [(4, 1, 0), (8, 2, 0), (16, 3, 0), (8, 64, 0)]:
+        got, f = steps(sp, c, prec, q0, tune)
+        assert np.array_equal(got, want), tune
+        assert halo_ok(c, f), tune
+    for upwind in (True, False):
+        e = conv_of(sp, n, upwind=upwind)
+        want, _ = steps(sp, e, prec, q0, (4, 8, 1), euler=True)
+        assert np.array_equal(steps(sp, e, prec, q0, (4, 2, 0), euler=True)[0], want)
+
+
+@pytest.mark.parametrize("n", [(144, 144, 144), (145, 144, 144), (100, 200, 151)])
+def test_default_path_on_both_sides_of_its_limit(sp, n):
+    """2.99M, 3.007M and 3.02M cells: direct kernel, pairs on 32 x 16 and on 64 x 8 tiles."""
+    q0 = gaussian_noise(*n, seed=6)
+    c = conv_of(sp, n)
+    a, b = c.field(), c.field()
+    c.upload(a, q0)
+    c.DoRK4(a, b, 0.0, 1e-4, 3)
+    assert np.array_equal(c.download(b), steps(sp, c, 0, q0, (4, 8, 1))[0])
+
+
+@pytest.mark.parametrize("prec,g", [("f64", "euler"), ("f32", "rk4")])
+def test_parareal_with_one_diffusivity_per_slice(sp, orc, prec, g):
+    n, slices = (18, 10, 7), 5
+    c = conv_of(sp, n, nufreq=40.0)
+    q0 = gaussian_noise(*n, seed=7)
+    f0, q, s = c.field(), c.field(), c.field()
+    c.upload(f0, q0)
+    conf = sp.RuntimeConfiguration(timeSlices=slices, nu0=0.02, nufreq=40.0, cy=-0.5, cz=0.25, gridSize=18,
+                                   endTime=5e-3, timeStepsFine=40, timeStepsCoarse=10, kmax=slices)
+    par = sp.Parareal(c, f0, q, 0.0, conf, coarse=g, coarse_precision=prec)
+    par.DoParallel()
+    # after as many iterations as slices the result is the serial fine run
+    c.DoRK4(f0, s, 0.0, conf.dtFine(), 40)
+    assert rel_l2(c.download(q), c.download(s)) < 1e-12
+    ref = orc.rk4(orc.params(n, dx=1.0 / 18, nu0=0.02, nufreq=40.0, cx=1.0, cy=-0.5, cz=0.25), q0, 0.0,
+                  conf.dtFine(), 40)
+    assert rel_l2(c.download(q), ref) < 1e-12
