@@ -269,11 +269,13 @@ long long sp_launch_count(void);
  * S1..S4, 4 = Euler): tile rows ty, z-chunk, kernel kind (0 direct loads, 1
  * TMA/mbarrier pipeline).  op 9 and 10: the fused stage pairs 1+2 and 3+4 of
  * FP64 RK4 steps: tile rows, planes per CTA (0 = one range per resident CTA),
- * kind 2 when RK4 steps run as fused pairs (4: on 32-column tiles), else 0.  Before
- * sp_autotune or sp_set_tune, a handle whose launches are small (up to 3M cells)
- * has pairs (kind 2) but runs the direct stage kernels (ops 0..3, kind 0) instead.
+ * kind 2 when RK4 steps run as fused pairs (4: on 32-column tiles), else 0.
  * op 11: kind 3 when FP64 RK4 propagations run cluster-resident on z-slabs
- * (sp_set_tune kind 3), 5 on (y,z) blocks (kind 5), else 0. */
+ * (sp_set_tune kind 3), 5 on (y,z) blocks (kind 5), else 0.
+ * Before sp_autotune or sp_set_tune, small FP64 launches do not take what ops 9..11
+ * show: up to about 36^3 cells per field they run cluster-resident where that is
+ * estimated to be faster, up to 3M cells in all on the direct stage kernels (ops
+ * 0..3, kind 0). */
 int sp_tuned_config(sp_convection* h, int precision, int batch, int op, int* ty, int* zchunk, int* kind);
 /* Runs the autotuner for this handle's grid at `batch` fields and precision: every
  * stage kernel gets the fastest of its candidate launch shapes, and FP64 RK4

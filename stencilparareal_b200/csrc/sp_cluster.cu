@@ -36,6 +36,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "sp_device.cuh"
@@ -55,19 +57,59 @@ struct ClusterArgs {
     long long item_stride, origin, px, plane;
     int ni, nj, nk;
     int nsteps;
-    const W13<double>* wtab;  // per-step weights (nu(t) varies) or null
-    W13<double> w;            // weights of every step when wtab is null
+    W13<double> w;            // weights of every step (one diffusivity)
+    const double* nutab;      // VARY: step i of item b takes nutab[i * items + b] ...
+    double nu[kClusterNuSteps];  // ... or (nutab null) nu[i]
+    int items;
+    double ca[3], s4;         // VARY: coefficients of R (Coef)
     double dthalf, dt, dt3, dt6;
     const int* item_lo;
     int item_base;
     int* err;
     StoreBounds sb;
+    double* in_images;        // where the images of the input go (the input field), or null
+    StoreBounds sb_in;
     int cy, cz;               // (y,z) blocks: CTAs per field along y and z
 };
 
+// The 13 weights for a diffusivity, with the roundings of fill_w13 on the host (no
+// contraction into FMAs), so that the fields equal the stage kernels' bit for bit.
+__device__ __forceinline__ void step_weights(W13<double>& w, const ClusterArgs& a, int step, int item) {
+    const double nu = a.nutab ? a.nutab[(long long)step * a.items + item] : a.nu[step];
+    const double nl = __dmul_rn(nu, a.s4), n16 = __dmul_rn(16., nl);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double c8 = __dmul_rn(8., a.ca[d]);
+        w.m1[d] = __dadd_rn(c8, n16);
+        w.p1[d] = __dadd_rn(-c8, n16);
+        w.m2[d] = __dadd_rn(-a.ca[d], -nl);
+        w.p2[d] = __dadd_rn(a.ca[d], -nl);
+    }
+    w.c = __dmul_rn(-90., nl);
+}
+
+// Periodic images of the cell pair (x, y, z) within two cells of a face -- on faces,
+// edges and corners, as Periodicity leaves them (p: the pair's address in its field).
+__device__ __forceinline__ void pair_images(const StoreBounds& b, double* p, const ClusterArgs& a, int x, int y, int z,
+                                            const V2& v) {
+#pragma unroll 1
+    for (int iz = 0; iz < 3; ++iz) {
+        if ((iz == 1 && z >= 2) || (iz == 2 && z < a.nk - 2)) continue;
+        double* pz = p + (iz == 0 ? 0 : (iz == 1 ? a.nk : -a.nk)) * a.plane;
+#pragma unroll 1
+        for (int iy = 0; iy < 3; ++iy) {
+            if ((iy == 1 && y >= 2) || (iy == 2 && y < a.nj - 2)) continue;
+            double* r = pz + (iy == 0 ? 0 : (iy == 1 ? a.nj : -a.nj)) * a.px;
+            if (iz | iy) gst16<double>(b, r, v);
+            if (x < 2) gst16<double>(b, r + a.ni, v);
+            if (x >= a.ni - 2) gst16<double>(b, r - a.ni, v);
+        }
+    }
+}
+
 // Cluster of C = nk / NZ CTAs per field (NZ >= 2, C >= 2); UPT units of two
 // x-adjacent cells of one row per thread, every own plane of each unit.
-template <int NZ, int UPT>
+template <int NZ, int UPT, bool VARY>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid_constant__ ClusterArgs a) {
     constexpr int NPL = NZ + 4;  // planes per buffer: 2 halo, NZ own, 2 halo
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -83,6 +125,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
     const uint32_t rank = cluster_rank();
     const int item = blockIdx.x / (int)C;
     // a converged Parareal slice: the whole cluster leaves before any cluster barrier
+    pdl_trigger();
+    pdl_wait();
     if (a.item_lo && item + a.item_base < *a.item_lo) return;
     const uint32_t lower = (rank + C - 1) % C, upper = (rank + 1) % C;
     const int z0 = (int)rank * NZ;
@@ -145,7 +189,13 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
             const int z = (z0 - 2 + p + nk) % nk;
             const V2 v = ld16<double>(fin + (long long)z * a.plane + (long long)uy[j] * a.px + ux[j]);
             sts2(base0 + (uint32_t)((p * plane_cells + uy[j] * ni + ux[j]) * 8), v);
-            if (p >= 2 && p < NZ + 2) q[j][p - 2] = v;
+            if (p >= 2 && p < NZ + 2) {
+                q[j][p - 2] = v;
+                if (a.in_images)
+                    pair_images(a.sb_in, a.in_images + (long long)item * a.item_stride + a.origin +
+                                             (long long)z * a.plane + (long long)uy[j] * a.px + ux[j],
+                                a, ux[j], uy[j], z, v);
+            }
         }
 #pragma unroll
     for (int j = 0; j < UPT; ++j)
@@ -156,7 +206,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
 
     bool bad = false;
     const int nstage = 4 * a.nsteps;
-    W13<double> w = a.w;
+    [[maybe_unused]] W13<double> wv;  // VARY: this step's weights; else they stay in the constant bank
+    const W13<double>& w = [&]() -> const W13<double>& {
+        if constexpr (VARY) return wv;
+        else return a.w;
+    }();
     // halo bytes per stage: two planes from each z-neighbour
     const uint32_t halo_bytes = 4u * (uint32_t)plane_cells * 8u;
     // stage g = 4 * step + ST reads buffer g & 1 and writes buffer (g + 1) & 1
@@ -269,20 +323,23 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
         __syncthreads();
     };
     for (int i = 0; i < a.nsteps; ++i) {
-        if (a.wtab) w = a.wtab[i];
+        if constexpr (VARY) step_weights(wv, a, i, item);
         stage(std::integral_constant<int, 0>{}, 4 * i);
         stage(std::integral_constant<int, 1>{}, 4 * i + 1);
         stage(std::integral_constant<int, 2>{}, 4 * i + 2);
         stage(std::integral_constant<int, 3>{}, 4 * i + 3);
     }
-    // result (the last stage's q') to global memory, interior only (the host
-    // fills the periodic images)
+    // result (the last stage's q') to global memory, with its periodic images
     double* fout = a.out + (long long)item * a.item_stride + a.origin;
 #pragma unroll
     for (int j = 0; j < UPT; ++j)
 #pragma unroll
         for (int o = 0; o < NZ; ++o)
-            if (uv[j]) gst16<double>(a.sb, fout + (long long)(z0 + o) * a.plane + (long long)uy[j] * a.px + ux[j], q[j][o]);
+            if (uv[j]) {
+                double* p = fout + (long long)(z0 + o) * a.plane + (long long)uy[j] * a.px + ux[j];
+                gst16<double>(a.sb, p, q[j][o]);
+                pair_images(a.sb, p, a, ux[j], uy[j], z0 + o, q[j][o]);
+            }
     if (__syncthreads_or(bad) && tid == 0) atomicExch(a.err, DEV_WAIT_TIMEOUT);
     cluster_sync_all();  // no CTA leaves while a neighbour may still address its shared memory
 }
@@ -307,7 +364,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
 // NT threads per CTA: 256 (up to 255 registers, one unit per thread) where the
 // block's units fit, else 512 (128 registers, up to two units per thread); at
 // 32^3 and 24^3 the 256-thread form is ~14 % faster, at 40^3 it would spill.
-template <int ZT, int UPT, int NT>
+template <int ZT, int UPT, int NT, bool VARY>
 __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__ ClusterArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);  // 2 mbarriers (stage parity)
@@ -328,6 +385,8 @@ __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__
     const uint32_t rank = cluster_rank();
     const int item = blockIdx.x / (int)C;
     // a converged Parareal slice: the whole cluster leaves before any cluster barrier
+    pdl_trigger();
+    pdl_wait();
     if (a.item_lo && item + a.item_base < *a.item_lo) return;
     const int ry = (int)rank % cy, rz = (int)rank / cy;
     const int y0 = ry * BY, z0 = rz * BZ;
@@ -389,16 +448,26 @@ __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__
 #pragma unroll
     for (int j = 0; j < UPT; ++j)
 #pragma unroll
-        for (int o = 0; o < ZT; ++o)
-            q[j][o] = uv[j] ? ld16<double>(fin + (long long)(z0 + uz[j] + o) * a.plane + (long long)(y0 + uy[j]) * a.px +
-                                           ux[j])
-                            : V2{};
+        for (int o = 0; o < ZT; ++o) {
+            q[j][o] = V2{};
+            if (!uv[j]) continue;
+            const int y = y0 + uy[j], z = z0 + uz[j] + o;
+            const long long at = (long long)z * a.plane + (long long)y * a.px + ux[j];
+            q[j][o] = ld16<double>(fin + at);
+            if (a.in_images)
+                pair_images(a.sb_in, a.in_images + (long long)item * a.item_stride + a.origin + at, a, ux[j], y, z,
+                            q[j][o]);
+        }
     __syncthreads();
     cluster_sync_all();  // every CTA runs and its barriers are initialised before any remote access
 
     bool bad = false;
     const int nstage = 4 * a.nsteps;
-    W13<double> w = a.w;
+    [[maybe_unused]] W13<double> wv;  // VARY: this step's weights; else they stay in the constant bank
+    const W13<double>& w = [&]() -> const W13<double>& {
+        if constexpr (VARY) return wv;
+        else return a.w;
+    }();
     const uint32_t halo_bytes = (uint32_t)(4 * BY + 4 * BZ) * row_bytes;
     const uint32_t yshift = (uint32_t)BY * row_bytes, zshift = (uint32_t)BZ * plane_bytes;
     auto stage = [&](auto stc, int g) {
@@ -485,7 +554,7 @@ __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__
         __syncthreads();
     };
     for (int i = 0; i < a.nsteps; ++i) {
-        if (a.wtab) w = a.wtab[i];
+        if constexpr (VARY) step_weights(wv, a, i, item);
         stage(std::integral_constant<int, 0>{}, 4 * i);
         stage(std::integral_constant<int, 1>{}, 4 * i + 1);
         stage(std::integral_constant<int, 2>{}, 4 * i + 2);
@@ -496,56 +565,58 @@ __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__
     for (int j = 0; j < UPT; ++j)
 #pragma unroll
         for (int o = 0; o < ZT; ++o)
-            if (uv[j])
-                gst16<double>(a.sb, fout + (long long)(z0 + uz[j] + o) * a.plane + (long long)(y0 + uy[j]) * a.px + ux[j],
-                              q[j][o]);
+            if (uv[j]) {
+                const int y = y0 + uy[j], z = z0 + uz[j] + o;
+                double* p = fout + (long long)z * a.plane + (long long)y * a.px + ux[j];
+                gst16<double>(a.sb, p, q[j][o]);
+                pair_images(a.sb, p, a, ux[j], y, z, q[j][o]);
+            }
     if (__syncthreads_or(bad) && tid == 0) atomicExch(a.err, DEV_WAIT_TIMEOUT);
     cluster_sync_all();  // no CTA leaves while a neighbour may still address its shared memory
 }
 
-template <int NZ, int UPT>
-size_t cluster_smem(const Geo& g) {
-    return 16 + (size_t)2 * (NZ + 4) * g.ni * g.nj * 8;
-}
-
-template <int NZ, int UPT>
-cudaError_t set_attr_cluster(const Geo* g) {
-    auto k = k_rk4_cluster<NZ, UPT>;
+template <typename K>
+cudaError_t set_attr_cluster(K k) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax);
-    (void)g;
     return e;
 }
 
-// Planes per CTA for a grid and batch: NZ in {2, 3, 4} with a cluster of at
-// most 16 CTAs whose buffers fit -- the smallest (the most CTAs per field: a
-// single field is bound by the latency of each stage) while the batch's CTAs
-// fit on the SMs at once, else the largest (fewer CTAs per field, more fields
-// at a time); 0 when the grid is not supported.
-int cluster_nz(const Geo& g, int items = 1) {
-    if (g.es != 8 || g.ni % 2 != 0 || g.ni < 4 || g.nj < 4 || g.nk < 4) return 0;
-    if ((long long)(g.ni / 2) * g.nj > 2LL * kClusterThreads) return 0;
-    int first = 0, last = 0;
-    for (int nz : {2, 3, 4}) {
-        if (g.nk % nz != 0) continue;
-        const int c = g.nk / nz;
-        if (c < 2 || c > 16) continue;
-        if (16 + (size_t)2 * (nz + 4) * g.ni * g.nj * 8 > (size_t)kClusterSmemMax) continue;
-        if (!first) first = nz;
-        last = nz;
-    }
-    if (!first) return 0;
-    return (long long)items * (g.nk / first) <= 148 ? first : last;
+// One cluster of C CTAs per field, with programmatic dependent launch.
+template <typename K>
+cudaError_t launch_clusters(K k, int C, int threads, size_t smem, const ClusterArgs& a, cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(C * a.items));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k, a);
 }
 
-template <int NZ, int UPT>
-cudaError_t launch_one(const Geo& g, const ClusterArgs& a, int items, cudaStream_t s) {
-    const int C = g.nk / NZ;
+// Clusters of C CTAs that run at once on the current device (0: none fits).  A
+// cluster lies inside one GPC, so of 148 SMs only 7 clusters of 16 find room, not 9.
+int resident_clusters(int C) {
+    static std::atomic<int> cached[64][17];  // zero-initialised; value + 1
+    int dev = 0;
+    if (C < 1 || C > 16 || cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const bool keep = dev >= 0 && dev < 64;
+    if (keep) {
+        const int v = cached[dev][C].load(std::memory_order_relaxed);
+        if (v) return v - 1;
+    }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(C * items));
+    cfg.gridDim = dim3((unsigned)C);
     cfg.blockDim = dim3(kClusterThreads);
-    cfg.dynamicSmemBytes = cluster_smem<NZ, UPT>(g);
-    cfg.stream = s;
+    cfg.dynamicSmemBytes = kClusterSmemMax;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)C;
@@ -553,29 +624,81 @@ cudaError_t launch_one(const Geo& g, const ClusterArgs& a, int items, cudaStream
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_rk4_cluster<NZ, UPT>, a);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_rk4_cluster<2, 1, false>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;  // asked again next time
+    }
+    if (keep) cached[dev][C].store(n + 1, std::memory_order_relaxed);
+    return n;
 }
 
-// (y,z) blocks for a grid and batch: cy, cz >= 2 with C = cy * cz <= 16, blocks
-// of at least 2 rows and 2 planes whose two buffers fit, and a thread form
-// (below).  Among those the one with the least estimated time: waves of CTAs
-// (one per SM) x (own cells + half the halo cells per CTA; at 32^3 the exchange
-// of a halo cell costs about half the stage work of an own cell), x 1.6 for the
-// spilling two-unit form; ties go to fewer units per thread.  cy = 0 when the
-// grid has no such blocks.
+// Estimated us per RK4 step of `items` fields on clusters of C CTAs that each own
+// `cells` cells and receive `halo` values per stage; a halo value costs about half
+// the work of a cell.  Fitted to 16^3 ... 40^3 (est. / measured): slabs 16^3 2.1 / 2.2,
+// 24^3 3.6 / 3.6, 32^3 5.7 / 6.3, 36^3 8.4 / 9.3, 40^3 12.0 / 13.1; blocks 16^3 1.5 /
+// 1.6, 32^3 4.5 / 4.5; 16 fields of 32^3 in blocks (3 waves) 13.4 / 14.1.
+double cluster_us(int C, int items, double cells, double halo) {
+    const int at_once = resident_clusters(C);
+    if (!at_once) return 1e30;
+    return (double)((items + at_once - 1) / at_once) * (0.95 + 1.15e-3 * (cells + 0.5 * halo));
+}
+
+// Planes per CTA for a grid and batch: the NZ in {2, 3, 4}, with a cluster of at
+// most 16 CTAs whose buffers fit, of the least estimated time; 0 when the grid is
+// not supported.
+int cluster_nz(const Geo& g, int items = 1, double* us = nullptr) {
+    if (g.es != 8 || g.ni % 2 != 0 || g.ni < 4 || g.nj < 4 || g.nk < 4) return 0;
+    if ((long long)(g.ni / 2) * g.nj > 2LL * kClusterThreads) return 0;
+    int best = 0;
+    double best_us = 0;
+    for (int nz : {2, 3, 4}) {
+        if (g.nk % nz != 0) continue;
+        const int c = g.nk / nz;
+        if (c < 2 || c > 16) continue;
+        if (16 + (size_t)2 * (nz + 4) * g.ni * g.nj * 8 > (size_t)kClusterSmemMax) continue;
+        const double t = cluster_us(c, items, (double)nz * g.ni * g.nj, 4. * g.ni * g.nj);
+        if (!best || t < best_us) {
+            best = nz;
+            best_us = t;
+        }
+    }
+    if (us) *us = best_us;
+    return best;
+}
+
+// f(<kernel>) for the slab kernel of NZ planes per CTA and UPT units per thread.
+template <bool VARY, typename F>
+cudaError_t with_slab_kernel(int nz, int upt, F&& f) {
+    switch (nz * 2 + upt - 1) {
+        case 4: return f(k_rk4_cluster<2, 1, VARY>);
+        case 5: return f(k_rk4_cluster<2, 2, VARY>);
+        case 6: return f(k_rk4_cluster<3, 1, VARY>);
+        case 7: return f(k_rk4_cluster<3, 2, VARY>);
+        case 8: return f(k_rk4_cluster<4, 1, VARY>);
+        case 9: return f(k_rk4_cluster<4, 2, VARY>);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 // bytes of shared memory per CTA of k_rk4_cluster2d: barriers, two buffers of
 // the block with its halo rows and planes, the accumulator of the own cells
 size_t cluster2d_smem(int ni, int by, int bz) {
     return 16 + (size_t)2 * (bz + 4) * (by + 4) * ni * 8 + (size_t)bz * by * ni * 8;
 }
 
+// (y,z) blocks for a grid and batch: cy, cz >= 2 with C = cy * cz <= 16, blocks
+// of at least 2 rows and 2 planes whose two buffers fit, and a thread form
+// (below).  Among those the one with the least estimated time, x 1.6 for the
+// spilling two-unit form; ties go to fewer units per thread.  cy = 0 when the
+// grid has no such blocks.
 struct Blocks2d {
     int cy = 0, cz = 0, zt = 0, upt = 0, nt = 0;
+    double us = 0;
 };
 Blocks2d blocks_2d(const Geo& g, int items) {
     Blocks2d best;
     if (g.es != 8 || g.ni % 2 != 0 || g.ni < 4 || g.nj < 4 || g.nk < 4 || items < 1) return best;
-    double best_cost = 0;
     for (int cy = 2; cy <= 8; ++cy)
         for (int cz = 2; cy * cz <= 16; ++cz) {
             if (g.nj % cy != 0 || g.nk % cz != 0) continue;
@@ -599,47 +722,50 @@ Blocks2d blocks_2d(const Geo& g, int items) {
                 nt = kClusterThreads;
                 if (upt > 2) continue;
             }
-            const long long ctas = (long long)items * cy * cz;
-            const long long waves = (ctas + 147) / 148;
             // the 512-thread form with two units per thread spills at its
             // 128-register cap: a batch of 16 fields of 32^3 ran its fine sweep
             // at 22.6 GCUPS on (2,4) blocks in one wave of that form, at 40.8 on
-            // (4,4) blocks in two waves of the 256-thread form
+            // (4,4) blocks of the 256-thread form
             const double form = nt == kClusterThreads && upt == 2 ? 1.6 : 1.0;
-            const double cost = form * (double)waves * ((double)g.ni * by * bz + 0.5 * (4.0 * by + 4.0 * bz) * g.ni);
-            if (!best.cy || cost < best_cost || (cost == best_cost && upt < best.upt)) {
-                best = Blocks2d{cy, cz, zt, upt, nt};
-                best_cost = cost;
-            }
+            const double us = cluster_us(cy * cz, items, form * g.ni * by * bz, form * (4.0 * by + 4.0 * bz) * g.ni);
+            if (!best.cy || us < best.us || (us == best.us && upt < best.upt))
+                best = Blocks2d{cy, cz, zt, upt, nt, us};
         }
     return best;
 }
 
-template <int ZT, int UPT, int NT>
-cudaError_t launch_one2d(const Geo& g, const Blocks2d& b, const ClusterArgs& a, int items, cudaStream_t s) {
-    auto k = k_rk4_cluster2d<ZT, UPT, NT>;
-    const int C = b.cy * b.cz;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(C * items));
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = cluster2d_smem(g.ni, g.nj / b.cy, g.nk / b.cz);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, a);
+// f(<kernel>) for the thread form of a block shape.
+template <bool VARY, typename F>
+cudaError_t with_block_kernel(int zt, int upt, int nt, F&& f) {
+    if (nt == 256) {
+        switch (zt) {
+            case 1: return f(k_rk4_cluster2d<1, 1, 256, VARY>);
+            case 2: return f(k_rk4_cluster2d<2, 1, 256, VARY>);
+            case 4: return f(k_rk4_cluster2d<4, 1, 256, VARY>);
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    switch (zt * 2 + upt - 1) {
+        case 2: return f(k_rk4_cluster2d<1, 1, 512, VARY>);
+        case 3: return f(k_rk4_cluster2d<1, 2, 512, VARY>);
+        case 4: return f(k_rk4_cluster2d<2, 1, 512, VARY>);
+        case 5: return f(k_rk4_cluster2d<2, 2, 512, VARY>);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
-template <int ZT, int UPT, int NT>
-cudaError_t set_attr_cluster2d() {
+template <bool VARY>
+cudaError_t prepare_cluster_kernels() {
+    auto set = [](auto k) { return set_attr_cluster(k); };
     cudaError_t e = cudaSuccess;
-    auto k = k_rk4_cluster2d<ZT, UPT, NT>;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax);
+    for (int nz = 2; nz <= 4; ++nz)
+        for (int upt = 1; upt <= 2; ++upt)
+            if (e == cudaSuccess) e = with_slab_kernel<VARY>(nz, upt, set);
+    for (int zt : {1, 2, 4})
+        if (e == cudaSuccess) e = with_block_kernel<VARY>(zt, 1, 256, set);
+    for (int zt = 1; zt <= 2; ++zt)
+        for (int upt = 1; upt <= 2; ++upt)
+            if (e == cudaSuccess) e = with_block_kernel<VARY>(zt, upt, 512, set);
     return e;
 }
 
@@ -649,24 +775,31 @@ bool cluster_supported(const Geo& g, int mode) {
     return mode == 2 ? blocks_2d(g, 1).cy != 0 : cluster_nz(g) != 0;
 }
 
+// Against the direct stage kernels, whose step takes about 9.5 us (four launches) +
+// 31 us per 1M cells: 32^3 10.7 us (cluster 4.5), 36^3 12.8 (9.3), 40^3 12.7 (13.1); 8
+// fields of 32^3 13.5 (9.4), 40 of them 48 (26), 8 of 40^3 27 (13.6).
+int default_cluster_mode(const Geo& g, int items) {
+    double slabs = 1e30;
+    if (!cluster_nz(g, items, &slabs)) slabs = 1e30;
+    const Blocks2d b = blocks_2d(g, items);
+    const double blocks = b.cy ? b.us : 1e30;
+    const double direct = 9.5 + 31e-6 * (double)g.ni * g.nj * g.nk * items;
+    if (std::min(slabs, blocks) >= direct) return 0;
+    return slabs < blocks ? 1 : 2;
+}
+
 cudaError_t prepare_cluster() {
-    cudaError_t e = cudaSuccess;
-    auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-    chk(set_attr_cluster<2, 1>(nullptr)); chk(set_attr_cluster<2, 2>(nullptr));
-    chk(set_attr_cluster<3, 1>(nullptr)); chk(set_attr_cluster<3, 2>(nullptr));
-    chk(set_attr_cluster<4, 1>(nullptr)); chk(set_attr_cluster<4, 2>(nullptr));
-    chk(set_attr_cluster2d<1, 1, 512>()); chk(set_attr_cluster2d<1, 2, 512>());
-    chk(set_attr_cluster2d<2, 1, 512>()); chk(set_attr_cluster2d<2, 2, 512>());
-    chk(set_attr_cluster2d<1, 1, 256>()); chk(set_attr_cluster2d<2, 1, 256>());
-    chk(set_attr_cluster2d<4, 1, 256>());
-    return e;
+    const cudaError_t e = prepare_cluster_kernels<false>();
+    return e != cudaSuccess ? e : prepare_cluster_kernels<true>();
 }
 
 cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_t s, int* err) {
     const int nz = L.mode == 2 ? 0 : cluster_nz(g, L.items);
     const Blocks2d b2 = L.mode == 2 ? blocks_2d(g, L.items) : Blocks2d{};
     if ((L.mode == 2 ? !b2.cy : !nz) || L.nsteps < 1 || L.items < 1) return cudaErrorInvalidValue;
-    ClusterArgs a;
+    if (!L.nutab && (L.nu_count < 1 || L.nu_count > kClusterNuSteps || (L.nu_count > 1 && L.nu_count < L.nsteps)))
+        return cudaErrorInvalidValue;
+    ClusterArgs a{};
     a.in = static_cast<const double*>(L.in);
     a.out = static_cast<double*>(L.out);
     a.item_stride = g.total;
@@ -675,8 +808,15 @@ cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_
     a.plane = g.plane;
     a.ni = g.ni; a.nj = g.nj; a.nk = g.nk;
     a.nsteps = L.nsteps;
-    a.wtab = static_cast<const W13<double>*>(L.wtab);
-    fill_w13(a.w, L.coef, L.nu);
+    a.items = L.items;
+    const bool vary = L.nutab || L.nu_count > 1;
+    if (!vary) fill_w13(a.w, L.coef, L.nu[0]);
+    a.nutab = L.nutab;
+    if (!L.nutab) std::copy(L.nu, L.nu + L.nu_count, a.nu);
+    for (int d = 0; d < 3; ++d) a.ca[d] = L.coef.ca[d];
+    a.s4 = L.coef.s4;
+    if (L.in != L.out) a.in_images = static_cast<double*>(L.in_images);
+    a.sb_in = out_bounds(a.in_images, g, L.items);
     a.dthalf = L.dt * .5;
     a.dt = L.dt;
     a.dt3 = L.dt / 3.;
@@ -687,34 +827,18 @@ cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_
     a.sb = out_bounds(L.out, g, L.items);
     a.cy = b2.cy;
     a.cz = b2.cz;
-    if (L.mode == 2) {
-        add_launches(1);
-        if (b2.nt == 256) {
-            if (b2.zt == 4) return launch_one2d<4, 1, 256>(g, b2, a, L.items, s);
-            if (b2.zt == 2) return launch_one2d<2, 1, 256>(g, b2, a, L.items, s);
-            return launch_one2d<1, 1, 256>(g, b2, a, L.items, s);
-        }
-        switch (b2.zt * 2 + b2.upt - 1) {
-            case 2: return launch_one2d<1, 1, 512>(g, b2, a, L.items, s);
-            case 3: return launch_one2d<1, 2, 512>(g, b2, a, L.items, s);
-            case 4: return launch_one2d<2, 1, 512>(g, b2, a, L.items, s);
-            default: return launch_one2d<2, 2, 512>(g, b2, a, L.items, s);
-        }
-    }
-    const bool two = (long long)(g.ni / 2) * g.nj > kClusterThreads;
     add_launches(1);
-    switch (nz * 2 + (two ? 1 : 0)) {
-        case 4: return launch_one<2, 1>(g, a, L.items, s);
-        case 5: return launch_one<2, 2>(g, a, L.items, s);
-        case 6: return launch_one<3, 1>(g, a, L.items, s);
-        case 7: return launch_one<3, 2>(g, a, L.items, s);
-        case 8: return launch_one<4, 1>(g, a, L.items, s);
-        default: return launch_one<4, 2>(g, a, L.items, s);
-    }
+    const int upt = (long long)(g.ni / 2) * g.nj > kClusterThreads ? 2 : 1;
+    auto launch = [&](auto k) {
+        return L.mode == 2 ? launch_clusters(k, b2.cy * b2.cz, b2.nt,
+                                             cluster2d_smem(g.ni, g.nj / b2.cy, g.nk / b2.cz), a, s)
+                           : launch_clusters(k, g.nk / nz, kClusterThreads,
+                                             16 + (size_t)2 * (nz + 4) * g.ni * g.nj * 8, a, s);
+    };
+    if (L.mode == 2)
+        return vary ? with_block_kernel<true>(b2.zt, b2.upt, b2.nt, launch)
+                    : with_block_kernel<false>(b2.zt, b2.upt, b2.nt, launch);
+    return vary ? with_slab_kernel<true>(nz, upt, launch) : with_slab_kernel<false>(nz, upt, launch);
 }
-
-void fill_cluster_weights(void* w13, const Coef& c, double nu) { fill_w13(*static_cast<W13<double>*>(w13), c, nu); }
-
-size_t cluster_weights_bytes() { return sizeof(W13<double>); }
 
 }  // namespace sp

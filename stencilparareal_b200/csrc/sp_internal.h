@@ -47,10 +47,15 @@ struct Tune {
     Shape op[kNumOps];
     Shape pair[2] = {Shape{8, 0, 1}, Shape{8, 0, 1}};  // fused stage pairs 1+2 and 3+4 (ty 8 or 16)
     int fused = 0;    // 1: FP64 RK4 steps run as the two fused pairs ...
-    int direct = 0;   // ... 1: except that launches this small run on the stage kernels of `op`
-    bool pairs() const { return fused && !direct; }
     int cluster = 0;  // FP64 RK4 propagations of small fields run cluster-resident (sp_cluster.cu):
                       // 1 on z-slabs, 2 on (y,z) blocks
+    // An untuned handle's choice for launches this small, before `fused` and `cluster`
+    // (which stay what sp_tuned_config reports):
+    int small_cluster = 0;  // cluster-resident, as `cluster`
+    int small_direct = 0;   // RK4 steps on the (direct) stage kernels of `op` instead of the pairs
+    int resident() const { return cluster ? cluster : small_cluster; }
+    bool pairs() const { return fused && !small_direct; }
+    void no_small() { small_cluster = small_direct = 0; }
     void set_all(const Shape& s) {
         for (auto& o : op) o = s;
     }
@@ -98,18 +103,21 @@ struct StageLaunch {
 
 // Many FP64 RK4 steps of small fields in one launch, each field held in the
 // distributed shared memory of one thread-block cluster (sp_cluster.cu).  Reads
-// the interiors of `items` fields at `in`, writes the interiors of the results
-// at `out` (in == out allowed; the periodic images of `out` are left to the
-// caller).  Step i uses the weights of `nu`, or wtab[i] (cluster_weights_bytes()
-// each, device memory) when wtab is set.
+// the interiors of `items` fields at `in`, writes the results with their periodic
+// images at `out` (in == out allowed).  Step i uses the diffusivity nu[i] (nu[0] in
+// every step if nu_count is 1), or nutab[i * items + b] for item b.
+constexpr int kClusterNuSteps = 256;
 struct ClusterLaunch {
     const void* in = nullptr;
     void* out = nullptr;
+    void* in_images = nullptr;       // the input field, if its periodic images are to be refreshed
     int items = 1;
     int nsteps = 0;
-    double dt = 0, nu = 0;
+    double dt = 0;
     Coef coef;
-    const void* wtab = nullptr;
+    int nu_count = 1;
+    const double* nu = nullptr;      // host, nu_count <= kClusterNuSteps values
+    const double* nutab = nullptr;   // device
     const int* item_lo = nullptr;    // as in StageLaunch
     int item_base = 0;
     int mode = 1;                    // 1: z-slabs (k_rk4_cluster), 2: (y,z) blocks (k_rk4_cluster2d)
@@ -117,10 +125,11 @@ struct ClusterLaunch {
 // mode 1: FP64, even ni, small planes, nk = C * {2,3,4} with 2 <= C <= 16;
 // mode 2: FP64, even ni, nj = cy * BY, nk = cz * BZ with cy, cz, BY, BZ >= 2, cy * cz <= 16
 bool cluster_supported(const Geo& g, int mode = 1);
+// The mode for launches of `items` fields before tuning, on the current device (0:
+// other paths are faster, or the grid or device has no cluster layout).
+int default_cluster_mode(const Geo& g, int items);
 cudaError_t prepare_cluster();
 cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_t s, int* err);
-size_t cluster_weights_bytes();
-void fill_cluster_weights(void* w13, const Coef& c, double nu);  // one entry of wtab (host memory)
 constexpr int kClusterSmemMax = 227 * 1024;
 
 // Launch shape of the single-stage kernels before tuning, for `items` fields per launch.

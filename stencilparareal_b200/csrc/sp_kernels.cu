@@ -901,50 +901,35 @@ cudaError_t launch_stage(const Geo& g, const StageLaunch& L, const Tune& t, cuda
 // ---------------------------------------------------------------------------
 // Pointwise kernels.
 
-// Periodicity: the three passes of Periodicity.cu:12-144 (I, then J over all I,
-// then K over all I and J), here for `items` fields.
+// Periodicity: what the three passes of Periodicity.cu:12-144 (I, then J over all
+// I, then K over all I and J) leave in the halo, here in one launch: every halo
+// cell is the interior cell at its wrapped indices, so nothing written is read.
+// A warp takes one row of the padded box, all of it outside the interior's rows,
+// the four x-halo cells inside.  The launches are what it costs (a call on 24^3
+// had three of ~2 us each in its chain).
 template <typename T>
-__global__ void k_period_i(T* f, Geo g, int items) {
-    const long long n = (long long)g.nj * g.nk * items;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(t % g.nj);
-        const int k = (int)((t / g.nj) % g.nk);
-        const int b = (int)(t / ((long long)g.nj * g.nk));
-        T* row = f + b * g.total + g.origin + (long long)k * g.plane + (long long)j * g.px;
-        row[-2] = row[g.ni - 2];
-        row[-1] = row[g.ni - 1];
-        row[g.ni] = row[0];
-        row[g.ni + 1] = row[1];
-    }
-}
-template <typename T>
-__global__ void k_period_j(T* f, Geo g, int items) {
-    const int wi = g.ni + 4;
-    const long long n = (long long)wi * g.nk * items;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % wi) - 2;
-        const int k = (int)((t / wi) % g.nk);
-        const int b = (int)(t / ((long long)wi * g.nk));
-        T* c = f + b * g.total + g.origin + (long long)k * g.plane + i;
-        c[-2 * g.px] = c[(long long)(g.nj - 2) * g.px];
-        c[-1 * g.px] = c[(long long)(g.nj - 1) * g.px];
-        c[(long long)g.nj * g.px] = c[0];
-        c[(long long)(g.nj + 1) * g.px] = c[g.px];
-    }
-}
-template <typename T>
-__global__ void k_period_k(T* f, Geo g, int items) {
-    const int wi = g.ni + 4, wj = g.nj + 4;
-    const long long n = (long long)wi * wj * items;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % wi) - 2;
-        const int j = (int)((t / wi) % wj) - 2;
-        const int b = (int)(t / ((long long)wi * wj));
-        T* c = f + b * g.total + g.origin + (long long)j * g.px + i;
-        c[-2 * g.plane] = c[(long long)(g.nk - 2) * g.plane];
-        c[-1 * g.plane] = c[(long long)(g.nk - 1) * g.plane];
-        c[(long long)g.nk * g.plane] = c[0];
-        c[(long long)(g.nk + 1) * g.plane] = c[g.plane];
+__global__ void __launch_bounds__(256) k_periodicity(T* f, Geo g) {
+    pdl_trigger();
+    pdl_wait();
+    const int rows_j = g.nj + 4;
+    const long long rows = (long long)rows_j * (g.nk + 4);
+    T* base = f + (long long)blockIdx.y * g.total + g.origin;
+    const int lane = threadIdx.x & 31;
+    for (long long r = blockIdx.x * 8LL + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8LL) {
+        const int k = (int)(r / rows_j) - 2, j = (int)(r % rows_j) - 2;
+        const int ks = k < 0 ? k + g.nk : (k >= g.nk ? k - g.nk : k);
+        const int js = j < 0 ? j + g.nj : (j >= g.nj ? j - g.nj : j);
+        T* dst = base + k * g.plane + j * g.px;
+        const T* src = base + ks * g.plane + js * g.px;
+        if (k == ks && j == js) {
+            if (lane < 4) {
+                const int x = lane < 2 ? lane - 2 : g.ni + lane - 2;
+                dst[x] = src[x < 0 ? x + g.ni : x - g.ni];
+            }
+        } else {
+            for (int x = lane - 2; x < g.ni + 2; x += 32)
+                dst[x] = src[x < 0 ? x + g.ni : (x >= g.ni ? x - g.ni : x)];
+        }
     }
 }
 
@@ -956,17 +941,11 @@ static unsigned grid_for(long long n, int block) {
 }
 
 cudaError_t launch_periodicity(const Geo& g, void* field, int items, cudaStream_t s) {
-    add_launches(3);
-    if (g.es == 8) {
-        k_period_i<double><<<grid_for((long long)g.nj * g.nk * items, 256), 256, 0, s>>>((double*)field, g, items);
-        k_period_j<double><<<grid_for((long long)(g.ni + 4) * g.nk * items, 256), 256, 0, s>>>((double*)field, g, items);
-        k_period_k<double><<<grid_for((long long)(g.ni + 4) * (g.nj + 4) * items, 256), 256, 0, s>>>((double*)field, g, items);
-    } else {
-        k_period_i<float><<<grid_for((long long)g.nj * g.nk * items, 256), 256, 0, s>>>((float*)field, g, items);
-        k_period_j<float><<<grid_for((long long)(g.ni + 4) * g.nk * items, 256), 256, 0, s>>>((float*)field, g, items);
-        k_period_k<float><<<grid_for((long long)(g.ni + 4) * (g.nj + 4) * items, 256), 256, 0, s>>>((float*)field, g, items);
-    }
-    return cudaGetLastError();
+    add_launches(1);
+    if (items < 1 || items > 65535) return cudaErrorInvalidValue;
+    const dim3 grid(grid_for((long long)(g.nj + 4) * (g.nk + 4), 8), (unsigned)items);
+    if (g.es == 8) return launch_pdl(k_periodicity<double>, grid, dim3(256), 0, s, static_cast<double*>(field), g);
+    return launch_pdl(k_periodicity<float>, grid, dim3(256), 0, s, static_cast<float*>(field), g);
 }
 
 // Adds the block's sums to acc[0 .. N-1] (and, for the maxima, takes the larger)

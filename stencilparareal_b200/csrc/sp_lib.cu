@@ -122,8 +122,8 @@ struct sp_convection {
     DevBuf red;         // reduction scratch (8 doubles)
     DevBuf dense;       // staging for the host-buffer entry point
     DevBuf adj_ckpt, adj_seg, adj_work, adj_par;  // adjoint workspace, kept between calls
-    DevBuf ctab;        // per-step stencil weights of the cluster-resident path (nu(t) varies)
-    std::map<std::tuple<int, int>, Tune> tunes;  // (prec, items) -> tune
+    std::map<std::tuple<int, int>, Tune> tunes;     // (prec, items) -> tune
+    std::map<std::tuple<int, int>, Tune> defaults;  // the same, before tuning
     std::map<std::tuple<int, const void*, double, double, int>, GraphEntry> graphs;
     cudaStream_t stream() const { return user ? user : own; }
     ~sp_convection() {
@@ -131,9 +131,21 @@ struct sp_convection {
             if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
         if (own) cudaStreamDestroy(own);
     }
+    // The launch shapes for `items` fields: set or tuned, else the defaults (worked
+    // out once).
     Tune tune(int prec, int items) {
         auto it = tunes.find({prec, items});
         if (it != tunes.end()) return it->second;
+        it = defaults.find({prec, items});
+        if (it != defaults.end()) return it->second;
+        int dev = device;
+        cudaGetDevice(&dev);
+        if (dev != device) cudaSetDevice(device);
+        const Tune t = default_tune(prec, items);
+        if (dev != device) cudaSetDevice(dev);
+        return defaults[{prec, items}] = t;
+    }
+    Tune default_tune(int prec, int items) const {
         const Shape sh = default_stage_shape(g[prec], items);
         Tune t;
         t.set_all(sh);
@@ -142,7 +154,8 @@ struct sp_convection {
         if (prec == 0 && pair_supported(g4)) {
             t.pair[0] = t.pair[1] = sh.tma ? default_pair_shape(g4, items) : Shape{8, 0, 1};
             t.fused = 1;
-            t.direct = sh.tma ? 0 : 1;
+            t.small_direct = sh.tma ? 0 : 1;
+            t.small_cluster = default_cluster_mode(g[0], items);
         }
         return t;
     }
@@ -384,34 +397,31 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
     cudaStream_t s = h->stream();
     int* err = h->err.as<int>();
     const Tune t = h->tune(prec, 1);
-    // Periodicity on the input, in place, as before the reference's first stencil.
-    SP_CUDA(launch_periodicity(g, const_cast<void*>(in), 1, s));
     const bool const_nu = h->P.nufreq == 0.;
-    if (rk && t.cluster && prec == 0 && cluster_supported(g, t.cluster) && (const_nu || !capturing(s))) {
-        // small field: every step in one launch, the field held in a cluster's
-        // shared memory (sp_cluster.cu); then the periodic images of `out`
+    const bool resident = rk && t.resident() && prec == 0 && cluster_supported(g, t.resident());
+    // Periodicity on the input, in place, as before the reference's first stencil
+    // (the cluster-resident path writes the images of its input itself).
+    if (!resident) SP_CUDA(launch_periodicity(g, const_cast<void*>(in), 1, s));
+    if (resident) {
+        // small field: all steps in one launch, the field held in a cluster's
+        // shared memory (sp_cluster.cu); with nu(tStart + i dt) (Convection.cpp:296-302)
+        // one launch per kClusterNuSteps steps, whose diffusivities are its arguments
         ClusterLaunch L;
-        L.mode = t.cluster;
-        L.in = in;
+        L.mode = t.resident();
         L.out = out;
-        L.nsteps = n;
         L.dt = dt;
         L.coef = h->coef;
-        L.nu = computenu(h->P.nu0, h->P.nufreq, tStart);
-        if (!const_nu) {
-            // nu(tStart + i dt) per step (Convection.cpp:296-302), as weights
-            const size_t wb = cluster_weights_bytes();
-            std::vector<unsigned char> tab((size_t)n * wb);
-            for (int i = 0; i < n; ++i)
-                fill_cluster_weights(tab.data() + (size_t)i * wb, h->coef,
-                                     computenu(h->P.nu0, h->P.nufreq, i == 0 ? tStart : tStart + i * dt));
-            if (h->ctab.alloc(tab.size()) != cudaSuccess) return fail(SP_ERR_NOMEM, "weight table");
-            SP_CUDA(cudaMemcpyAsync(h->ctab.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, s));
-            SP_CUDA(cudaStreamSynchronize(s));  // the host table goes out of scope
-            L.wtab = h->ctab.p;
+        double nus[kClusterNuSteps];
+        L.nu = nus;
+        for (int i = 0; i < n; i += L.nsteps) {
+            L.in = i == 0 ? in : out;
+            L.in_images = i == 0 ? const_cast<void*>(in) : nullptr;
+            L.nsteps = const_nu ? n : std::min(n - i, kClusterNuSteps);
+            L.nu_count = const_nu ? 1 : L.nsteps;
+            for (int k = 0; k < L.nu_count; ++k)
+                nus[k] = computenu(h->P.nu0, h->P.nufreq, i + k == 0 ? tStart : tStart + (i + k) * dt);
+            SP_CUDA(launch_rk4_cluster(g, L, s, err));
         }
-        SP_CUDA(launch_rk4_cluster(g, L, s, err));
-        SP_CUDA(launch_periodicity(g, out, 1, s));
     } else if (rk && t.pairs() && prec == 0 && pair_supported(h->g4)) {
         // fused stage pairs: widen the input once, alternate the step-start
         // field between wbuf(0) and wbuf(1), write the last step to `out`
@@ -571,6 +581,7 @@ int sp_set_tune(sp_convection* h, int precision, int batch, int ty, int zchunk, 
                                                     "cy x cz <= 16, whose buffers fit in shared memory");
         Tune t = h->tune(precision, batch);
         t.cluster = kind == 3 ? 1 : 2;
+        t.no_small();
         h->tunes[{precision, batch}] = t;
         h->drop_graphs();
         return SP_OK;
@@ -589,7 +600,8 @@ int sp_set_tune(sp_convection* h, int precision, int batch, int ty, int zchunk, 
         sh.tx = kind == 4 ? 32 : 64;
         t.pair[0] = t.pair[1] = sh;
         t.fused = 1;
-        t.direct = 0;
+        t.cluster = 0;
+        t.no_small();
         h->tunes[{precision, batch}] = t;
         h->drop_graphs();
         return SP_OK;
@@ -936,7 +948,8 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
     }
     // fused stage pairs (FP64): best shape per pair, then fused or single-stage
     // steps by timing whole steps of both paths
-    best.fused = best.direct = 0;
+    best.fused = best.cluster = 0;
+    best.no_small();
     if (precision == SP_F64 && pair_supported(h->g4)) {
         const Geo& g4 = h->g4;
         const size_t wb = (size_t)batch * g4.total * g4.es;
@@ -1087,7 +1100,6 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
     // small fields: the cluster-resident paths (z-slabs, (y,z) blocks) against
     // the best of the above, timed as they are used (a DoRK4 of a graph chunk of
     // steps for one field; four batched steps for a batch)
-    best.cluster = 0;
     if (precision == SP_F64 && (cluster_supported(g, 1) || cluster_supported(g, 2))) {
         int* err = h->err.as<int>();
         float path_ms[3] = {1e30f, 1e30f, 1e30f};
@@ -1105,7 +1117,7 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
                 if (c) {
                     ClusterLaunch L;
                     L.mode = c;
-                    L.in = p; L.out = p; L.items = batch; L.nsteps = 4; L.dt = dtt; L.nu = nu; L.coef = h->coef;
+                    L.in = p; L.out = p; L.items = batch; L.nsteps = 4; L.dt = dtt; L.nu = &nu; L.coef = h->coef;
                     x = launch_rk4_cluster(g, L, s, err);
                 } else {
                     for (int i = 0; i < 4 && x == cudaSuccess; ++i)
@@ -1355,8 +1367,8 @@ int enqueue_coarse(sp_parareal* pr, const void* src, const Geo& gsrc, double t0,
 // (small fields), fused stage pairs, or the four stage kernels per step.
 bool cluster_sweep(const sp_parareal* pr) {
     sp_convection* h = pr->prop;
-    const int mode = h->tune(0, pr->P).cluster;
-    return h->P.nufreq == 0. && mode && cluster_supported(pr->g64, mode);
+    const int mode = h->tune(0, pr->P).resident();
+    return mode && cluster_supported(pr->g64, mode);
 }
 bool fused_sweep(const sp_parareal* pr) {
     sp_convection* h = pr->prop;
@@ -1405,17 +1417,17 @@ int emit_iteration(sp_parareal* pr, cudaStream_t s, bool events, int parts, int 
     if (cluster && (parts & 1) && e == cudaSuccess) {
         // every fine step of every iterating slice in one launch, each slice in one cluster
         ClusterLaunch L;
-        L.mode = tf.cluster;
+        L.mode = tf.resident();
         L.in = pr->u(0);
         L.out = pr->f(0);
         L.items = P;
         L.nsteps = pr->tsF;
         L.dt = pr->dtF;
-        L.nu = h->P.nu0;
+        L.nu = &h->P.nu0;
+        if (!const_nu) L.nutab = pr->nutab.as<double>();
         L.coef = h->coef;
         L.item_lo = pr->itemlo();
         e = launch_rk4_cluster(g, L, s, err);
-        if (e == cudaSuccess) e = launch_periodicity(g, pr->f(0), P, s);
     }
     if (fused && (parts & 1)) {
         // widen the slice inputs once, alternate step start / accumulator

@@ -5,6 +5,7 @@ thread-block cluster, split into z-slabs (tune kind 3) or into (y,z) blocks
 (same operations, same order) and the oracle's to 1e-12."""
 import numpy as np
 import pytest
+import torch
 
 from ics import fourier_modes, gaussian_noise, rel_l2
 
@@ -138,3 +139,32 @@ def test_parareal_fine_sweep_on_clusters_equals_stage_kernels(sp, skip, P, kind)
         outs.append((conv.download(fsol), rep["iterations"]))
     assert np.array_equal(outs[0][0], outs[1][0])
     assert outs[0][1] == outs[1][1] == 4
+
+
+@pytest.mark.parametrize("n,P,nufreq", [((32, 32, 32), 1, 0.0), ((36, 36, 36), 1, 0.0), ((22, 26, 30), 1, 30.0),
+                                        ((16, 16, 16), 20, 0.0), ((24, 24, 24), 9, 60.0), ((40, 40, 40), 8, 0.0),
+                                        ((31, 32, 32), 1, 0.0)])
+def test_default_small_path_equals_stage_kernels(sp, n, P, nufreq):
+    """What an untuned handle runs for small fields (slabs, blocks, several waves of
+    clusters, one diffusivity per step or slice, an odd width on the direct kernel)."""
+    q0 = gaussian_noise(*n, seed=4)
+    got = []
+    for stages in (False, True):
+        conv = _conv(sp, n, nufreq=nufreq)
+        if stages:
+            conv.set_tune(sp.SP_F64, P, 4, 8, 1)
+            conv.set_tune(sp.SP_F64, 1, 4, 8, 1)
+        a, b = conv.field(), conv.field()
+        conv.upload(a, q0)
+        if P == 1:  # 270 steps: more than one launch's table of diffusivities
+            conv.DoRK4(a, b, 0.1, 1e-5, 270)
+        else:
+            conf = sp.RuntimeConfiguration(timeSlices=P, nu0=0.02, nufreq=nufreq, gridSize=n[0], endTime=1e-3,
+                                           timeStepsFine=6 * P, timeStepsCoarse=P, kmax=3)
+            sp.Parareal(conv, a, b, 0.0, conf, coarse="rk4", coarse_precision="f32").DoParallel()
+        conv.Periodicity(b)  # both halos as Periodicity leaves them
+        got.append((conv.download(b), a.data.clone(), b.data.clone()))
+    exact = P == 1 or nufreq == 0.0  # one diffusivity per slice: the stage kernels sum in another order
+    assert np.array_equal(got[0][0], got[1][0]) if exact else rel_l2(got[0][0], got[1][0]) < 1e-13
+    if P == 1:  # the input's halo was refreshed in place
+        assert torch.equal(got[0][1], got[1][1])
