@@ -62,7 +62,6 @@ struct PairArgs {
     int span;          // planes of the flattened (tile group, z) space per group (total < 2^31)
     const int* item_lo;
     int item_base;
-    W13<double> w;
     double c1y;        // first stage:  y = c1y k + base
     double c2y, c2a;   // second stage: y = c2y k + q (pair 1+2), acc / result = c2a k + base
     double* yout;      // pair 1+2: y2 (internal geometry, images 4 deep)
@@ -154,10 +153,11 @@ struct PairShape {
     static constexpr size_t smem = 128 + (size_t)(NSQ * SB + NE * SE + NP * SP) * 8 + (NSQ + NP) * 8;
 };
 
-template <int PAIR, int TY, int NSQ, int NP, int TXP = 64>
+template <int PAIR, int TY, int NSQ, int NP, int TXP, int NW>
 __global__ void __launch_bounds__(TY * TXP / 2, TY * TXP / 2 <= 256 ? 2 : 1)
     k_rk4_pair(const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_q,
-               const __grid_constant__ CUtensorMap tm_a, const PairArgs a) {
+               const __grid_constant__ CUtensorMap tm_a, const PairArgs a,
+               const __grid_constant__ Weights<double, NW> wt) {
     using S = PairShape<TY, NSQ, NP, PAIR, TXP>;
     constexpr int TX = S::TX, WB = S::WB, WE = S::WE, SB = S::SB, SE = S::SE, SP = S::SP;
     constexpr int NE = S::NE, NHR = S::NHR, NH = S::NH;
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(TY * TXP / 2, TY * TXP / 2 <= 256 ? 2 : 1)
             // the centre value is the window's)
             {
                 double k[2];
-                rhs_s<WB>(a.w, S2 + m_s8, qw[(K + 2) % 5], qw[K], qw[(K + 1) % 5], qw[(K + 3) % 5], qw[(K + 4) % 5], k);
+                rhs_s<WB>(wt.w[NW == 1 ? 0 : b], S2 + m_s8, qw[(K + 2) % 5], qw[K], qw[(K + 1) % 5], qw[(K + 3) % 5], qw[(K + 4) % 5], k);
                 V2 en;
                 if constexpr (PAIR == 0) {
                     const V2& c = qw[(K + 2) % 5];
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(TY * TXP / 2, TY * TXP / 2 <= 256 ? 2 : 1)
                     cen = lds2(S2 + h_s8);
                 }
                 double k[2];
-                rhs_s<WB>(a.w, S2 + h_s8, cen, zm2, zm1, zp1, zp2, k);
+                rhs_s<WB>(wt.w[NW == 1 ? 0 : b], S2 + h_s8, cen, zm2, zm1, zp1, zp2, k);
                 V2 base = cen, hv;
                 if constexpr (PAIR == 1) base = lds2(PW + h_e8);
 #pragma unroll
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(TY * TXP / 2, TY * TXP / 2 <= 256 ? 2 : 1)
             // second stage on plane z0-4+v (first-stage plane v-2, stencil plane v)
             if (v >= 4) {
                 double k[2];
-                rhs_s<WE>(a.w, E2 + m_e8, ew[(K + 3) % 5], ew[(K + 1) % 5], ew[(K + 2) % 5], ew[(K + 4) % 5], ew[K], k);
+                rhs_s<WE>(wt.w[NW == 1 ? 0 : b], E2 + m_e8, ew[(K + 3) % 5], ew[(K + 1) % 5], ew[(K + 2) % 5], ew[(K + 4) % 5], ew[K], k);
                 V2 o;
                 [[maybe_unused]] V2 oa;
                 if constexpr (PAIR == 0) {
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kColX * kColY)
     });
 }
 
-template <int PAIR, int TY, int NSQ, int NP, int TXP>
+template <int PAIR, int NW, int TY, int NSQ, int NP, int TXP>
 cudaError_t launch_pair_T(const Geo& g4, const Geo& go, const PairLaunch& L, const Shape& sh, cudaStream_t s,
                           int* err) {
     using S = PairShape<TY, NSQ, NP, PAIR, TXP>;
@@ -534,7 +534,7 @@ cudaError_t launch_pair_T(const Geo& g4, const Geo& go, const PairLaunch& L, con
         if (ctas_dev == 0) {
             int sms = 0, occ = 0;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rk4_pair<PAIR, TY, NSQ, NP, TXP>, S::NT, S::smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rk4_pair<PAIR, TY, NSQ, NP, TXP, NW>, S::NT, S::smem);
             ctas_dev = std::max(1, sms) * std::max(1, occ);
             if (dev >= 0 && dev < 64) cached[dev].store(ctas_dev, std::memory_order_relaxed);
         }
@@ -543,7 +543,8 @@ cudaError_t launch_pair_T(const Geo& g4, const Geo& go, const PairLaunch& L, con
     }
     a.item_lo = L.item_lo;
     a.item_base = L.item_base;
-    fill_w13<double>(a.w, L.coef, L.nu);
+    Weights<double, NW> wt;
+    fill_weights(wt, L.coef, L.nu, L.nu_items, L.items);
     const double dthalf = L.dt * .5;
     if (PAIR == 0) {  // the coefficients of stages 1 and 2 of the single-stage path
         a.c1y = dthalf; a.c2y = dthalf; a.c2a = L.dt / 3.;
@@ -562,13 +563,31 @@ cudaError_t launch_pair_T(const Geo& g4, const Geo& go, const PairLaunch& L, con
     const long long nct = (total + a.span - 1) / a.span * a.cy;
     if (nct > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const dim3 grid((unsigned)nct);
-    return launch_pdl(k_rk4_pair<PAIR, TY, NSQ, NP, TXP>, grid, dim3(S::NT), S::smem, s, ts, tq, ta, a);
+    return launch_pdl(k_rk4_pair<PAIR, TY, NSQ, NP, TXP, NW>, grid, dim3(S::NT), S::smem, s, ts, tq, ta, a, wt);
 }
 
-template <int PAIR, int TY, int NSQ, int NP, int TXP = 64>
+template <int PAIR, int NW, int TY, int NSQ, int NP, int TXP>
 cudaError_t set_pair_attr() {
-    return cudaFuncSetAttribute(k_rk4_pair<PAIR, TY, NSQ, NP, TXP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_rk4_pair<PAIR, TY, NSQ, NP, TXP, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)PairShape<TY, NSQ, NP, PAIR, TXP>::smem);
+}
+template <int PAIR, int NW>
+cudaError_t set_pair_attrs() {
+    cudaError_t e = set_pair_attr<PAIR, NW, 8, 7, 2, 64>();
+    if (e == cudaSuccess) e = set_pair_attr<PAIR, NW, 16, 7, 2, 64>();
+    if (e == cudaSuccess) e = set_pair_attr<PAIR, NW, 16, 7, 2, 32>();
+    return e;
+}
+
+// tile 64 x 8, 64 x 16 (one row per warp) or 32 x 16 (two rows per warp)
+template <int PAIR, int NW>
+cudaError_t launch_pair_shape(const Geo& g4, const Geo& go, const PairLaunch& L, const Shape& sh, cudaStream_t s,
+                              int* err) {
+    add_launches(1);
+    if (sh.tx == 32 && sh.ty == 16) return launch_pair_T<PAIR, NW, 16, 7, 2, 32>(g4, go, L, sh, s, err);
+    if (sh.tx == 64 && sh.ty == 8) return launch_pair_T<PAIR, NW, 8, 7, 2, 64>(g4, go, L, sh, s, err);
+    if (sh.tx == 64 && sh.ty == 16) return launch_pair_T<PAIR, NW, 16, 7, 2, 64>(g4, go, L, sh, s, err);
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace
@@ -584,12 +603,10 @@ unsigned long long take_store_violations_pairs() {
 }
 
 cudaError_t prepare_pairs() {
-    cudaError_t e = set_pair_attr<0, 8, 7, 2>();
-    if (e == cudaSuccess) e = set_pair_attr<1, 8, 7, 2>();
-    if (e == cudaSuccess) e = set_pair_attr<0, 16, 7, 2>();
-    if (e == cudaSuccess) e = set_pair_attr<1, 16, 7, 2>();
-    if (e == cudaSuccess) e = set_pair_attr<0, 16, 7, 2, 32>();
-    if (e == cudaSuccess) e = set_pair_attr<1, 16, 7, 2, 32>();
+    cudaError_t e = set_pair_attrs<0, 1>();
+    if (e == cudaSuccess) e = set_pair_attrs<1, 1>();
+    if (e == cudaSuccess) e = set_pair_attrs<0, kItemWeights>();
+    if (e == cudaSuccess) e = set_pair_attrs<1, kItemWeights>();
     return e;
 }
 
@@ -618,21 +635,25 @@ Shape default_pair_shape(const Geo& g, int items) {
 
 cudaError_t launch_pair(const Geo& g4, const Geo& go, const PairLaunch& L, const Shape& sh, cudaStream_t s,
                         int* err) {
-    add_launches(1);
     if (!pair_supported(g4) || g4.halo != 4 || sh.zchunk < 0) return cudaErrorInvalidValue;
-    // tile 64 x 8, 64 x 16 (one row per warp) or 32 x 16 (two rows per warp)
-    const bool narrow = sh.tx == 32;
-    if (narrow && sh.ty != 16) return cudaErrorInvalidValue;
-    if (L.pair == 0) {
-        if (narrow) return launch_pair_T<0, 16, 7, 2, 32>(g4, go, L, sh, s, err);
-        if (sh.ty == 8) return launch_pair_T<0, 8, 7, 2, 64>(g4, go, L, sh, s, err);
-        if (sh.ty == 16) return launch_pair_T<0, 16, 7, 2, 64>(g4, go, L, sh, s, err);
-    } else {
-        if (narrow) return launch_pair_T<1, 16, 7, 2, 32>(g4, go, L, sh, s, err);
-        if (sh.ty == 8) return launch_pair_T<1, 8, 7, 2, 64>(g4, go, L, sh, s, err);
-        if (sh.ty == 16) return launch_pair_T<1, 16, 7, 2, 64>(g4, go, L, sh, s, err);
+    if (!L.nu_items)
+        return L.pair == 0 ? launch_pair_shape<0, 1>(g4, go, L, sh, s, err)
+                           : launch_pair_shape<1, 1>(g4, go, L, sh, s, err);
+    for (int b = 0; b < L.items; b += kItemWeights) {  // as many items per launch as it has weights for
+        PairLaunch l = L;
+        const size_t at = (size_t)b * g4.total;
+        l.items = std::min(kItemWeights, L.items - b);
+        l.nu_items = L.nu_items + b;
+        l.item_base = L.item_base + b;
+        l.q = static_cast<const double*>(L.q) + at;
+        l.y2 = static_cast<double*>(L.y2) + at;
+        l.acc = static_cast<double*>(L.acc) + at;
+        if (L.pair == 1) l.out = static_cast<double*>(L.out) + (size_t)b * go.total;
+        const cudaError_t e = L.pair == 0 ? launch_pair_shape<0, kItemWeights>(g4, go, l, sh, s, err)
+                                          : launch_pair_shape<1, kItemWeights>(g4, go, l, sh, s, err);
+        if (e != cudaSuccess) return e;
     }
-    return cudaErrorInvalidValue;
+    return cudaSuccess;
 }
 
 cudaError_t launch_widen(const Geo& g4, void* dst, const Geo& gs, const void* src, int items, const int* item_lo,

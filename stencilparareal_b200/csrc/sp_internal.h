@@ -87,7 +87,7 @@ struct StageLaunch {
     const int* item_lo = nullptr;    // device word: items below it are skipped (may be null)
     int item_base = 0;               // index of item 0 in the item_lo numbering
     double nu = 0;                   // diffusivity (all items) ...
-    const double* nu_items = nullptr;// ... or one value per item (device)
+    const double* nu_items = nullptr;// ... or one value per item (host; FP64 RK stages)
     double c_y = 0, c_acc = 0;       // stage coefficients
     Coef coef;
     // adjoint extras
@@ -135,6 +135,10 @@ constexpr int kClusterSmemMax = 227 * 1024;
 // Launch shape of the single-stage kernels before tuning, for `items` fields per launch.
 Shape default_stage_shape(const Geo& g, int items, bool adjoint = false);
 
+// Items with a diffusivity of their own that one launch takes (their weights are
+// kernel arguments, 104 bytes each: within 4 KB); larger batches take several.
+constexpr int kItemWeights = 32;
+
 // Launches one stage kernel; counts the launch.  err: device error word.
 cudaError_t launch_stage(const Geo& g, const StageLaunch& L, const Tune& t, cudaStream_t s, int* err);
 
@@ -152,7 +156,8 @@ struct PairLaunch {
     int items = 1;
     const int* item_lo = nullptr;    // as in StageLaunch
     int item_base = 0;
-    double nu = 0, dt = 0;
+    double nu = 0, dt = 0;           // diffusivity of all items ...
+    const double* nu_items = nullptr;// ... or one value per item (host)
     Coef coef;
 };
 bool pair_supported(const Geo& g);  // FP64, at least 4 interior cells per dimension

@@ -18,9 +18,8 @@
 // plus nu * Laplace4 (ConvectionFunctions.h:135-167), written as
 //   R = sum_d c_d/(12dx) * (8(q[-1]-q[+1]) - (q[-2]-q[+2]))_d
 //     + nu/(12dx^2) * (16 S1 - S2 - 90 q),  S1/S2 = sums of the +-1/+-2 neighbours,
-// the same coefficients regrouped into differences (the adjoint, and RK stages
-// with one diffusivity per item); the other RK stages use them combined into 13
-// per-offset weights (rhs_w13, sp_stencil.cuh), as the fused stage pairs do.  R2 is RHS2Stage
+// the same coefficients regrouped into differences (the adjoint); the RK
+// stages of both implementations use them combined into 13 per-offset weights (rhs_w13, sp_stencil.cuh), as the fused stage pairs do.  R2 is RHS2Stage
 // (Convection.cpp:30-55) with the upwind Advection2 (ConvectionFunctions.h:18-42).
 //
 // Fields carry a 2-cell halo (layout in include/sp_abi.h).  Every kernel that
@@ -112,14 +111,11 @@ struct KArgs {
     T ca0, ca1, ca2;          // c_d/(12dx)
     T u0, u1, u2;             // RHS2 advection coefficients
     int m0, m1, m2;           // RHS2 difference modes
-    double nu;                // diffusivity (when nu_items is null)
-    const double* nu_items;   // per-item diffusivity
-    double lap_scale;         // 1/(12dx^2) (RHS4) or 1/dx^2 (RHS2)
+    T nl;                     // nu/(12dx^2) (adjoint) or nu/dx^2 (Euler)
     T c_y, c_acc;             // stage coefficients
     T sigma;                  // adjoint: mu_s = sigma * (stencil input)
     double* par_acc;          // adjoint: 4 parameter-gradient sums
     double gs_nu, gs_c;       // adjoint: scales of the nu and c sums
-    W13<T> w;                 // RHS4 weights for the launch's nu (TMA RK stages)
     int* err;
 };
 
@@ -158,10 +154,10 @@ __device__ __forceinline__ void rk_update(const KArgs<T>& a, T k, T c, T q0, T q
     (void)q0; (void)q1; (void)oa;
 }
 
-// One cell of one stage.  p0..p2: pointwise operands; oy/oa: outputs;
+// One cell of an Euler or adjoint stage.  p0..p2: pointwise operands; oy/oa: outputs;
 // g[4]: adjoint parameter partial sums (unscaled).
 template <typename T, int OP>
-__device__ __forceinline__ void cell_op(const KArgs<T>& a, T nl, const Nb<T>& s, T p0, T p1, T p2, T& oy, T& oa,
+__device__ __forceinline__ void cell_op(const KArgs<T>& a, const Nb<T>& s, T p0, T p1, T p2, T& oy, T& oa,
                                         double* g, bool live) {
     if constexpr (OP == OP_EULER) {
         const T dqx = diff_mode(a.m0, s.c, s.xm1, s.xp1);
@@ -177,7 +173,7 @@ __device__ __forceinline__ void cell_op(const KArgs<T>& a, T nl, const Nb<T>& s,
         } else {
             lap = ((s.xm1 + s.xp1) + (s.ym1 + s.yp1) + (s.zm1 + s.zp1)) - T(6) * s.c;
         }
-        const T k = fmaT(nl, lap, adv);
+        const T k = fmaT(a.nl, lap, adv);
         oy = fmaT(a.c_y, k, s.c);
         (void)p0; (void)p1; (void)p2; (void)oa; (void)g; (void)live;
     } else {
@@ -198,13 +194,9 @@ __device__ __forceinline__ void cell_op(const KArgs<T>& a, T nl, const Nb<T>& s,
             lap = fmaT(T(-90), s.c, fmaT(T(16), S1, -S2));
         }
         const T adv = fmaT(a.ca0, ax, fmaT(a.ca1, ay, a.ca2 * az));
-        if constexpr (!OpTraits<OP>::adjoint) {
-            const T k = fmaT(nl, lap, adv);
-            rk_update<T, OP>(a, k, s.c, p0, p1, oy, oa);
-            (void)g; (void)live;
-        } else {
+        {
             // R^T m = -sum_d c_d D_d m + nu L m (D_d antisymmetric, L symmetric on the periodic grid)
-            const T ybar = a.sigma * fmaT(nl, lap, -adv);
+            const T ybar = a.sigma * fmaT(a.nl, lap, -adv);
             if (live) {
                 g[0] += (double)p0 * (double)lap;
                 g[1] += (double)p0 * (double)ax;
@@ -254,12 +246,6 @@ __device__ __forceinline__ void store_images_vec(T* base, int x, int y, int z, c
     if (y >= a.nj - 2) put_vec<T, N>(b, row - (long long)a.nj * a.px, x, a.ni, v);
     if (z < 2) put_vec<T, N>(b, row + (long long)a.nk * a.plane, x, a.ni, v);
     if (z >= a.nk - 2) put_vec<T, N>(b, row - (long long)a.nk * a.plane, x, a.ni, v);
-}
-
-template <typename T>
-__device__ __forceinline__ T item_nl(const KArgs<T>& a, int b) {
-    const double nu = a.nu_items ? a.nu_items[b] : a.nu;
-    return (T)(nu * a.lap_scale);
 }
 
 // Reduces the four adjoint parameter sums over the CTA (warp shuffles, then
@@ -320,8 +306,9 @@ __device__ __forceinline__ T* after_wait(T* p) {
     return p;
 }
 
-template <typename T, int OP, bool PER_ITEM>
-__global__ void __launch_bounds__(512) k_stage_direct(const __grid_constant__ KArgs<T> a) {
+template <typename T, int OP, int NW>
+__global__ void __launch_bounds__(512)
+    k_stage_direct(const __grid_constant__ KArgs<T> a, const __grid_constant__ Weights<T, NW> wt) {
     constexpr int N = V16<T>::N, NPW = OpTraits<OP>::npw;
     constexpr bool RK = OP <= OP_RK_S4;
     using V = Vec<T, N>;
@@ -343,7 +330,6 @@ __global__ void __launch_bounds__(512) k_stage_direct(const __grid_constant__ KA
         if constexpr (NPW > 0) pw[0] = after_wait(a.pw0) + col;
         if constexpr (NPW > 1) pw[1] = after_wait(a.pw1) + col;
         if constexpr (NPW > 2) pw[2] = after_wait(a.pw2) + col;
-        const T nl = item_nl(a, b);
         const long long pl = a.plane, px = a.px;
         V win[5];  // the column's planes z-2 .. z+2
 #pragma unroll
@@ -375,8 +361,8 @@ __global__ void __launch_bounds__(512) k_stage_direct(const __grid_constant__ KA
                 if constexpr (NPW > 0) q0 = p[0].v[e];
                 if constexpr (NPW > 1) q1 = p[1].v[e];
                 if constexpr (NPW > 2) q2 = p[2].v[e];
-                if constexpr (RK && !PER_ITEM) rk_update<T, OP>(a, rhs_w13(a.w, s), s.c, q0, q1, vy, va);
-                else cell_op<T, OP>(a, nl, s, q0, q1, q2, vy, va, g, x + e < a.ni);
+                if constexpr (RK) rk_update<T, OP>(a, rhs_w13(wt.w[NW == 1 ? 0 : b], s), s.c, q0, q1, vy, va);
+                else cell_op<T, OP>(a, s, q0, q1, q2, vy, va, g, x + e < a.ni);
                 oy.v[e] = vy;
                 oa.v[e] = va;
             }
@@ -402,11 +388,11 @@ __global__ void __launch_bounds__(512) k_stage_direct(const __grid_constant__ KA
 // except on the four planes next to the z faces.
 
 
-template <typename T, int OP, int TY, int NS, int NP>
+template <typename T, int OP, int TY, int NS, int NP, int NW>
 __global__ void __launch_bounds__(32 * TY)
     k_stage_tma(const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_p0,
                 const __grid_constant__ CUtensorMap tm_p1, const __grid_constant__ CUtensorMap tm_p2,
-                const KArgs<T> a) {
+                const KArgs<T> a, const __grid_constant__ Weights<T, NW> wt) {
     constexpr int VX = V16<T>::N;
     constexpr int TX = 32 * VX;
     constexpr int LX = VX;
@@ -518,7 +504,6 @@ __global__ void __launch_bounds__(32 * TY)
         for (int t = z0 - 2 + NS; t <= z0 - 1 + NS && t <= ylast; ++t) { issue_y(t); y_hi = t; }
     }
 
-    const T nl = item_nl(a, b);
     const int y = y0 + w;
     const int x = x0 + lane * VX;
     const bool live = y < a.nj && x < a.ni;
@@ -579,9 +564,9 @@ __global__ void __launch_bounds__(32 * TY)
             if constexpr (NPA > 2) q2 = p2v.v[e];
             T vy = 0, va = 0;
             if constexpr (RK) {
-                rk_update<T, OP>(a, rhs_w13(a.w, s), s.c, q0, q1, vy, va);
+                rk_update<T, OP>(a, rhs_w13(wt.w[NW == 1 ? 0 : b], s), s.c, q0, q1, vy, va);
             } else {
-                cell_op<T, OP>(a, nl, s, q0, q1, q2, vy, va, g, live && x + e < a.ni);
+                cell_op<T, OP>(a, s, q0, q1, q2, vy, va, g, live && x + e < a.ni);
             }
             oy.v[e] = vy;
             oa.v[e] = va;
@@ -680,15 +665,13 @@ KArgs<T> make_args(const Geo& g, const StageLaunch& L, const Shape& t, int* err)
     a.ca0 = (T)c.ca[0]; a.ca1 = (T)c.ca[1]; a.ca2 = (T)c.ca[2];
     a.u0 = (T)c.u[0]; a.u1 = (T)c.u[1]; a.u2 = (T)c.u[2];
     a.m0 = c.mode[0]; a.m1 = c.mode[1]; a.m2 = c.mode[2];
-    a.nu = L.nu; a.nu_items = L.nu_items;
-    a.lap_scale = (L.op == OP_EULER) ? c.s2 : c.s4;
+    a.nl = (T)(L.nu * (L.op == OP_EULER ? c.s2 : c.s4));
     a.c_y = (T)L.c_y; a.c_acc = (T)L.c_acc;
     a.err = err;
     // RK4 stages alternate the sweep direction (S1, S3 descending; S2, S4 ascending),
     // so that each stage starts on the planes the previous one touched last
     a.zrev = (L.op == OP_RK_S1 || L.op == OP_RK_S3) ? 1 : 0;
     a.sb_y = out_bounds(L.yout, g, L.items);
-    fill_w13<T>(a.w, c, L.nu);  // RHS4 as per-offset weights (TMA RK stages; one nu per launch)
     switch (L.op) {
         case OP_RK_S1: break;
         case OP_RK_S2: a.aout = (T*)L.acc; a.pw0 = (const T*)L.q; break;
@@ -715,17 +698,17 @@ KArgs<T> make_args(const Geo& g, const StageLaunch& L, const Shape& t, int* err)
     return a;
 }
 
-template <typename T, int OP>
-cudaError_t launch_direct_T(const Geo& g, KArgs<T> a, const Shape& t, int items, cudaStream_t s) {
+template <typename T, int OP, int NW>
+cudaError_t launch_direct_T(const Geo& g, const StageLaunch& L, KArgs<T> a, const Shape& t, cudaStream_t s) {
     if (t.ty != 4 && t.ty != 8 && t.ty != 16) return cudaErrorInvalidValue;
     const unsigned threads = 32u * (unsigned)t.ty;
     a.tiles_x = (g.ni + V16<T>::N - 1) / V16<T>::N;
     const long long chunks = (long long)a.tiles_x * g.nj;
-    const dim3 grid((unsigned)((chunks + threads - 1) / threads), (unsigned)a.nzc, (unsigned)items);
+    const dim3 grid((unsigned)((chunks + threads - 1) / threads), (unsigned)a.nzc, (unsigned)L.items);
     if (chunks > 0x7fffffffLL || grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
-    if constexpr (OP <= OP_RK_S4)
-        if (a.nu_items) return launch_pdl(k_stage_direct<T, OP, true>, grid, dim3(threads), 0, s, a);
-    return launch_pdl(k_stage_direct<T, OP, false>, grid, dim3(threads), 0, s, a);
+    Weights<T, NW> wt;
+    fill_weights(wt, L.coef, L.nu, L.nu_items, L.items);
+    return launch_pdl(k_stage_direct<T, OP, NW>, grid, dim3(threads), 0, s, a, wt);
 }
 
 template <typename T, int OP, int TY, int NS, int NP>
@@ -735,7 +718,7 @@ size_t tma_smem_bytes() {
     return 128 + (size_t)NS * W * H * sizeof(T) + (size_t)NP * NPA * TX * TY * sizeof(T) + (NS + NP) * 8;
 }
 
-template <typename T, int OP, int TY, int NS, int NP>
+template <typename T, int OP, int NW, int TY, int NS, int NP>
 cudaError_t launch_tma_T(const Geo& g, const StageLaunch& L, KArgs<T> a, const Shape& t, cudaStream_t s) {
     constexpr int VX = V16<T>::N, TX = 32 * VX, W = TX + 2 * VX, H = TY + 4;
     CUtensorMap ts{}, t0{}, t1{}, t2{};
@@ -749,66 +732,71 @@ cudaError_t launch_tma_T(const Geo& g, const StageLaunch& L, KArgs<T> a, const S
     dim3 grid(a.tiles_x * tiles_y, a.nzc, L.items);
     if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
     const size_t smem = tma_smem_bytes<T, OP, TY, NS, NP>();
-    return launch_pdl(k_stage_tma<T, OP, TY, NS, NP>, grid, dim3(32 * TY), smem, s, ts, t0, t1, t2, a);
+    Weights<T, NW> wt;
+    fill_weights(wt, L.coef, L.nu, L.nu_items, L.items);
+    return launch_pdl(k_stage_tma<T, OP, TY, NS, NP, NW>, grid, dim3(32 * TY), smem, s, ts, t0, t1, t2, a, wt);
 }
 
-template <typename T, int OP, int TY, int NS, int NP>
+template <typename T, int OP, int NW, int TY, int NS, int NP>
 cudaError_t set_attr_T() {
-    return cudaFuncSetAttribute(k_stage_tma<T, OP, TY, NS, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_stage_tma<T, OP, TY, NS, NP, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)tma_smem_bytes<T, OP, TY, NS, NP>());
 }
 
-template <typename T, int OP>
+template <typename T, int OP, int NW = 1>
 cudaError_t set_attr_op() {
-    cudaError_t e = set_attr_T<T, OP, 4, 5, 3>();
-    if (e == cudaSuccess) e = set_attr_T<T, OP, 8, 5, 3>();
-    if (e == cudaSuccess) e = set_attr_T<T, OP, 16, 4, 2>();
+    cudaError_t e = set_attr_T<T, OP, NW, 4, 5, 3>();
+    if (e == cudaSuccess) e = set_attr_T<T, OP, NW, 8, 5, 3>();
+    if (e == cudaSuccess) e = set_attr_T<T, OP, NW, 16, 4, 2>();
     return e;
 }
 
 
 // Ring depths per tile height: NS stencil slots (prefetch NS-3 planes ahead),
 // NP pointwise slots (prefetch NP-1 planes ahead).
-template <typename T, int OP>
-cudaError_t launch_tma_op(const Geo& g, const StageLaunch& L, const KArgs<T>& a, const Shape& t, cudaStream_t s) {
+template <typename T, int OP, int NW>
+cudaError_t launch_op(const Geo& g, const StageLaunch& L, const Shape& t, cudaStream_t s, int* err) {
+    const KArgs<T> a = make_args<T>(g, L, t, err);
+    if (!t.tma) return launch_direct_T<T, OP, NW>(g, L, a, t, s);
     switch (t.ty) {
-        case 4: return launch_tma_T<T, OP, 4, 5, 3>(g, L, a, t, s);
-        case 8: return launch_tma_T<T, OP, 8, 5, 3>(g, L, a, t, s);
-        case 16: return launch_tma_T<T, OP, 16, 4, 2>(g, L, a, t, s);
+        case 4: return launch_tma_T<T, OP, NW, 4, 5, 3>(g, L, a, t, s);
+        case 8: return launch_tma_T<T, OP, NW, 8, 5, 3>(g, L, a, t, s);
+        case 16: return launch_tma_T<T, OP, NW, 16, 4, 2>(g, L, a, t, s);
         default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename T>
-cudaError_t launch_T(const Geo& g, const StageLaunch& L, Shape t, cudaStream_t s, int* err) {
-    // one diffusivity per item (batched slices with nufreq != 0): direct kernel, on
-    // its own shape where the given one is the TMA ring's (16 fields of 64^3: 149
-    // us per step against 161 on 4 rows x 8 planes)
-    const bool tma = t.tma && !L.nu_items;
-    if (t.tma && !tma) t = Shape{8, 4, 0};
-    KArgs<T> a = make_args<T>(g, L, t, err);
-#define SP_OPCASE(OPV)                                                              \
-    case OPV:                                                                       \
-        return tma ? launch_tma_op<T, OPV>(g, L, a, t, s)                           \
-                   : launch_direct_T<T, OPV>(g, a, t, L.items, s);
+cudaError_t launch_T(const Geo& g, const StageLaunch& L, const Shape& t, cudaStream_t s, int* err) {
+    if constexpr (sizeof(T) == 8) {
+        switch (L.nu_items ? L.op : -1) {
+            case -1: break;
+            case OP_RK_S1: return launch_op<T, OP_RK_S1, kItemWeights>(g, L, t, s, err);
+            case OP_RK_S2: return launch_op<T, OP_RK_S2, kItemWeights>(g, L, t, s, err);
+            case OP_RK_S3: return launch_op<T, OP_RK_S3, kItemWeights>(g, L, t, s, err);
+            case OP_RK_S4: return launch_op<T, OP_RK_S4, kItemWeights>(g, L, t, s, err);
+            default: return cudaErrorInvalidValue;
+        }
+    } else if (L.nu_items) {
+        return cudaErrorInvalidValue;
+    }
     switch (L.op) {
-        SP_OPCASE(OP_RK_S1)
-        SP_OPCASE(OP_RK_S2)
-        SP_OPCASE(OP_RK_S3)
-        SP_OPCASE(OP_RK_S4)
-        SP_OPCASE(OP_EULER)
+        case OP_RK_S1: return launch_op<T, OP_RK_S1, 1>(g, L, t, s, err);
+        case OP_RK_S2: return launch_op<T, OP_RK_S2, 1>(g, L, t, s, err);
+        case OP_RK_S3: return launch_op<T, OP_RK_S3, 1>(g, L, t, s, err);
+        case OP_RK_S4: return launch_op<T, OP_RK_S4, 1>(g, L, t, s, err);
+        case OP_EULER: return launch_op<T, OP_EULER, 1>(g, L, t, s, err);
         default: break;
     }
     if constexpr (sizeof(T) == 8) {
         switch (L.op) {
-            SP_OPCASE(OP_ADJ + 0)
-            SP_OPCASE(OP_ADJ + 1)
-            SP_OPCASE(OP_ADJ + 2)
-            SP_OPCASE(OP_ADJ + 3)
+            case OP_ADJ + 0: return launch_op<T, OP_ADJ + 0, 1>(g, L, t, s, err);
+            case OP_ADJ + 1: return launch_op<T, OP_ADJ + 1, 1>(g, L, t, s, err);
+            case OP_ADJ + 2: return launch_op<T, OP_ADJ + 2, 1>(g, L, t, s, err);
+            case OP_ADJ + 3: return launch_op<T, OP_ADJ + 3, 1>(g, L, t, s, err);
             default: break;
         }
     }
-#undef SP_OPCASE
     return cudaErrorInvalidValue;
 }
 
@@ -828,6 +816,8 @@ cudaError_t prepare_kernels() {
     chk(set_attr_op<double, OP_RK_S1>()); chk(set_attr_op<double, OP_RK_S2>());
     chk(set_attr_op<double, OP_RK_S3>()); chk(set_attr_op<double, OP_RK_S4>());
     chk(set_attr_op<double, OP_EULER>());
+    chk(set_attr_op<double, OP_RK_S1, kItemWeights>()); chk(set_attr_op<double, OP_RK_S2, kItemWeights>());
+    chk(set_attr_op<double, OP_RK_S3, kItemWeights>()); chk(set_attr_op<double, OP_RK_S4, kItemWeights>());
     chk(set_attr_op<double, OP_ADJ + 0>()); chk(set_attr_op<double, OP_ADJ + 1>());
     chk(set_attr_op<double, OP_ADJ + 2>()); chk(set_attr_op<double, OP_ADJ + 3>());
     chk(set_attr_op<float, OP_RK_S1>()); chk(set_attr_op<float, OP_RK_S2>());
@@ -891,11 +881,24 @@ Shape default_stage_shape(const Geo& g, int items, bool adjoint) {
 }
 
 cudaError_t launch_stage(const Geo& g, const StageLaunch& L, const Tune& t, cudaStream_t s, int* err) {
-    add_launches(1);
     if (L.op < 0 || L.op >= kNumOps) return cudaErrorInvalidValue;
     const Shape& sh = t.op[L.op];
-    if (L.prec == 0) return launch_T<double>(g, L, sh, s, err);
-    return launch_T<float>(g, L, sh, s, err);
+    auto launch = [&](const StageLaunch& l) {
+        add_launches(1);
+        return l.prec == 0 ? launch_T<double>(g, l, sh, s, err) : launch_T<float>(g, l, sh, s, err);
+    };
+    if (!L.nu_items || L.items <= kItemWeights) return launch(L);
+    for (int b = 0; b < L.items; b += kItemWeights) {
+        StageLaunch l = L;
+        auto at = [&](auto* p) { return p ? (decltype(p))((const char*)p + (size_t)b * g.total * g.es) : p; };
+        l.items = std::min(kItemWeights, L.items - b);
+        l.nu_items = L.nu_items + b;
+        l.item_base = L.item_base + b;
+        l.yin = at(L.yin); l.q = at(L.q); l.acc = at(L.acc); l.yout = at(L.yout);
+        const cudaError_t e = launch(l);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------

@@ -1287,7 +1287,8 @@ struct sp_parareal {
     DevBuf D;              // P+1 coarse fields: slice increments (increment form)
     DevBuf Gt;             // 2 coarse fields (coarse result / ping-pong) + 3 coarse scratch
     DevBuf ctl;            // device control: item_lo (int) + defect sums (2P doubles) + err4
-    DevBuf nutab;          // fine nu table (tsF x P) when nufreq != 0
+    std::vector<double> nus;  // fine nu table (tsF x P) when nufreq != 0 ...
+    DevBuf nutab;             // ... and its copy for the cluster-resident path
     int* h_itemlo = nullptr;   // pinned
     double* h_def = nullptr;   // pinned, 2P + 4
     cudaGraphExec_t iter = nullptr;
@@ -1372,7 +1373,7 @@ bool cluster_sweep(const sp_parareal* pr) {
 }
 bool fused_sweep(const sp_parareal* pr) {
     sp_convection* h = pr->prop;
-    return !cluster_sweep(pr) && h->P.nufreq == 0. && h->tune(0, pr->P).pairs() && pair_supported(h->g4);
+    return !cluster_sweep(pr) && h->tune(0, pr->P).pairs() && pair_supported(h->g4);
 }
 
 // Allocates the fine-sweep scratch of the path the tune selects; must run
@@ -1404,7 +1405,7 @@ int emit_iteration(sp_parareal* pr, cudaStream_t s, bool events, int parts, int 
     const Tune tf = h->tune(0, P);
     int* err = h->err.as<int>();
     const bool const_nu = h->P.nufreq == 0.;
-    // F sweep as fused stage pairs when the tune says so and one nu serves all slices
+    // F sweep as fused stage pairs when the tune says so
     const bool fused = fused_sweep(pr);
     const Geo& g4 = h->g4;
     const size_t fstride = (size_t)P * g.total;
@@ -1447,6 +1448,7 @@ int emit_iteration(sp_parareal* pr, cudaStream_t s, bool events, int parts, int 
             double* Q = (i % 2) ? W1 : W0;
             double* A = (i % 2) ? W0 : W1;
             const bool last = i + 1 == pr->tsF;
+            if (!const_nu) L.nu_items = pr->nus.data() + (size_t)i * P;
             L.pair = 0; L.q = Q; L.y2 = WY; L.acc = A;
             e = launch_pair(g4, g4, L, tf.pair[0], s, err);
             L.pair = 1; L.out = last ? (void*)pr->f(0) : (void*)A;
@@ -1456,7 +1458,7 @@ int emit_iteration(sp_parareal* pr, cudaStream_t s, bool events, int parts, int 
     for (int i = 0; i < pr->tsF && e == cudaSuccess && (parts & 1) && !fused && !cluster; ++i) {
         NuSrc nu;
         if (const_nu) nu.nu = h->P.nu0;
-        else nu.items = pr->nutab.as<double>() + (size_t)i * P;
+        else nu.items = pr->nus.data() + (size_t)i * P;
         const void* in = i == 0 ? (const void*)pr->u(0) : (const void*)pr->f(0);
         e = enqueue_rk4_step(g, 0, h->coef, pr->dtF, nu, in, pr->f(0), ya, yb, acc, P, pr->itemlo(), 0, tf, s, err);
     }
@@ -1706,7 +1708,8 @@ int sp_parareal_create(sp_convection* prop, const sp_parareal_cfg* cfg, sp_parar
         // nu(t) per slice and fine step (Convection.h:81-84) with the time
         // sequence of DoRK4 (Convection.cpp:296-302) or of the split first
         // step of the asynchronous variant (Parareal.h:119-124).
-        std::vector<double> tab((size_t)pr->tsF * P);
+        std::vector<double>& tab = pr->nus;
+        tab.resize((size_t)pr->tsF * P);
         for (int r = 0; r < P; ++r) {
             const double tStart = pr->slice * (pr->first + r);
             const double tStartFine = tStart + pr->dtF;

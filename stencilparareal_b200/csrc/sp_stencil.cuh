@@ -34,6 +34,25 @@ inline void fill_w13(W13<T>& w, const Coef& c, double nu) {
     w.c = (T)(-90. * nl);
 }
 
+// The weights of a launch, a kernel argument of its own: one set, or (NW > 1) one per
+// item of the batch.  Read from the constant bank with the block's item as the
+// index they cost no registers (pairs 122, TMA stages 64-72, the same as with one
+// set), so a batch with one diffusivity per slice runs the kernels of a uniform one.
+template <typename T, int NW>
+struct Weights {
+    W13<T> w[NW];
+};
+template <typename T, int NW>
+inline void fill_weights(Weights<T, NW>& out, const Coef& c, double nu, const double* nu_items, int items) {
+    if constexpr (NW == 1) {
+        (void)nu_items; (void)items;
+        fill_w13<T>(out.w[0], c, nu);
+    } else {
+        (void)nu;
+        for (int b = 0; b < items && b < NW; ++b) fill_w13<T>(out.w[b], c, nu_items[b]);
+    }
+}
+
 // The 13 stencil operands of one cell.
 template <typename T>
 struct Nb {

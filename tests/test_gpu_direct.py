@@ -2,8 +2,8 @@
 the TMA rings and the fused pairs.
 
 All of them evaluate the RK4 stages (and Euler) with the same operations in the
-same order, so the fields must agree bit for bit; with one diffusivity per slice
-the direct kernel sums in another order and is held to the oracle.
+same order, so the fields must agree bit for bit, with one diffusivity for all
+slices or one per slice.
 """
 import numpy as np
 import pytest
@@ -74,20 +74,23 @@ def test_default_path_on_both_sides_of_its_limit(sp, n):
     assert np.array_equal(c.download(b), steps(sp, c, 0, q0, (4, 8, 1))[0])
 
 
-@pytest.mark.parametrize("prec,g", [("f64", "euler"), ("f32", "rk4")])
-def test_parareal_with_one_diffusivity_per_slice(sp, orc, prec, g):
-    n, slices = (18, 10, 7), 5
-    c = conv_of(sp, n, nufreq=40.0)
+@pytest.mark.parametrize("slices", [5, 32, 33, 70])
+def test_parareal_with_one_diffusivity_per_slice(sp, orc, slices):
+    """Every path takes one set of weights per slice, at most 32 per launch."""
+    n, total = (18, 10, 7), 4 * slices
     q0 = gaussian_noise(*n, seed=7)
-    f0, q, s = c.field(), c.field(), c.field()
-    c.upload(f0, q0)
     conf = sp.RuntimeConfiguration(timeSlices=slices, nu0=0.02, nufreq=40.0, cy=-0.5, cz=0.25, gridSize=18,
-                                   endTime=5e-3, timeStepsFine=40, timeStepsCoarse=10, kmax=slices)
-    par = sp.Parareal(c, f0, q, 0.0, conf, coarse=g, coarse_precision=prec)
-    par.DoParallel()
-    # after as many iterations as slices the result is the serial fine run
-    c.DoRK4(f0, s, 0.0, conf.dtFine(), 40)
-    assert rel_l2(c.download(q), c.download(s)) < 1e-12
-    ref = orc.rk4(orc.params(n, dx=1.0 / 18, nu0=0.02, nufreq=40.0, cx=1.0, cy=-0.5, cz=0.25), q0, 0.0,
-                  conf.dtFine(), 40)
-    assert rel_l2(c.download(q), ref) < 1e-12
+                                   endTime=1e-4 * total, timeStepsFine=total, timeStepsCoarse=2 * slices, kmax=2)
+    got = []
+    # direct, TMA ring, pairs on both tile widths
+    for tune in [(8, 2, 0), (4, 3, 1), (8, 3, 2), (16, 0, 4)]:
+        c = conv_of(sp, n, nufreq=40.0)
+        c.set_tune(sp.SP_F64, slices, *tune)
+        f0, q = c.field(), c.field()
+        c.upload(f0, q0)
+        sp.Parareal(c, f0, q, 0.0, conf).DoParallel()
+        got.append(c.download(q))
+        assert np.array_equal(got[0], got[-1]), tune
+    p = orc.params(n, dx=1.0 / 18, nu0=0.02, nufreq=40.0, cx=1.0, cy=-0.5, cz=0.25)
+    cfg = orc.parareal_cfg(1e-4 * total, slices, total, 2 * slices, 2)
+    assert rel_l2(got[0], orc.parareal(p, cfg, q0)[0]) < 1e-11
