@@ -274,8 +274,8 @@ long long sp_launch_count(void);
  * (sp_set_tune kind 3), 5 on (y,z) blocks (kind 5), else 0.
  * Before sp_autotune or sp_set_tune, small FP64 launches do not take what ops 9..11
  * show: up to about 36^3 cells per field they run cluster-resident where that is
- * estimated to be faster, up to 3M cells in all on the direct stage kernels (ops
- * 0..3, kind 0). */
+ * estimated to be faster, up to 3M cells in all (more where the pairs' tiles fit the
+ * grid badly) on the stage kernels (ops 0..3, kind 0 or 1). */
 int sp_tuned_config(sp_convection* h, int precision, int batch, int op, int* ty, int* zchunk, int* kind);
 /* Runs the autotuner for this handle's grid at `batch` fields and precision: every
  * stage kernel gets the fastest of its candidate launch shapes, and FP64 RK4

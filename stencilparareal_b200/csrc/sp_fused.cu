@@ -610,22 +610,41 @@ cudaError_t prepare_pairs() {
     return e;
 }
 
+namespace {
+// Cells of a plane covered by tiles of tx x ty.
+long long padded(const Geo& g, int tx, int ty) {
+    return (long long)((g.ni + tx - 1) / tx) * tx * ((g.nj + ty - 1) / ty) * ty;
+}
+}  // namespace
+
+// Beyond the direct kernel's sizes, pairs and TMA stage kernels (tiles of 64 x 4)
+// cost about the same per cell of their tiles (20-22 us per 1M cells and step)
+// until the stages' traffic (104 against 56 B per cell) leaves the L2, so the tile
+// that pads the plane less decides: 8 fields of 100^3 202 us per step on the stages
+// (128 x 100 cells) against 237 (128 x 104), 8 of 96^3 190 (128 x 96) against 162
+// (96 x 96).  With equal tiles the stages win while a launch is short (16 fields of
+// 64^3 113 / 120, 2 of 128^3 101 / 110, 4 of 128^3 189 / 186), the pairs beyond (256^3
+// 315 / 338).
+bool stages_before_pairs(const Geo& g, int items) {
+    const double cells = (double)g.ni * g.nj * g.nk * items;
+    const double pairs = (double)std::min(padded(g, 32, 16), padded(g, 64, 8));
+    const double weight = cells <= 5e6 ? 0.93 : (cells <= 12e6 ? 1.01 : 1.1);
+    return weight * (double)padded(g, 64, 4) < pairs;
+}
+
 // Tiles of 32 x 16 cells with as many z-ranges as fill two waves of CTAs (two per
 // SM), no range longer than 64 planes -- or 64 x 8 over one range per resident CTA
 // where those pad the plane less.  us per step, 32 x 16 / 64 x 8: 192^3 (24 planes)
 // 155 / 158, 256^3 (64 planes) 315 / 325, 8 fields of 96^3 161 / 212; 8 of 100^3
 // (128 x 112 against 128 x 104 cells) 244 / 235.
 Shape default_pair_shape(const Geo& g, int items) {
-    auto padded = [&](int tx, int ty) {
-        return (long long)((g.ni + tx - 1) / tx) * tx * ((g.nj + ty - 1) / ty) * ty;
-    };
     Shape sh;
-    if (padded(64, 8) < padded(32, 16)) {
+    if (padded(g, 64, 8) < padded(g, 32, 16)) {
         sh.ty = 8;
         sh.zchunk = 0;
         return sh;
     }
-    const long long tiles = padded(32, 16) / 512 * items;
+    const long long tiles = padded(g, 32, 16) / 512 * items;
     const long long ranges = std::max((g.nk + 63) / 64LL, std::max(1LL, 4 * 148 / tiles));
     sh.tx = 32;
     sh.ty = 16;

@@ -52,10 +52,10 @@ struct Tune {
     // An untuned handle's choice for launches this small, before `fused` and `cluster`
     // (which stay what sp_tuned_config reports):
     int small_cluster = 0;  // cluster-resident, as `cluster`
-    int small_direct = 0;   // RK4 steps on the (direct) stage kernels of `op` instead of the pairs
+    int small_stages = 0;   // RK4 steps on the stage kernels of `op` instead of the pairs
     int resident() const { return cluster ? cluster : small_cluster; }
-    bool pairs() const { return fused && !small_direct; }
-    void no_small() { small_cluster = small_direct = 0; }
+    bool pairs() const { return fused && !small_stages; }
+    void no_small() { small_cluster = small_stages = 0; }
     void set_all(const Shape& s) {
         for (auto& o : op) o = s;
     }
@@ -161,7 +161,9 @@ struct PairLaunch {
     Coef coef;
 };
 bool pair_supported(const Geo& g);  // FP64, at least 4 interior cells per dimension
-Shape default_pair_shape(const Geo& g, int items);  // before tuning
+// Before tuning: the pairs' shape, and whether FP64 steps run on the stage kernels instead.
+Shape default_pair_shape(const Geo& g, int items);
+bool stages_before_pairs(const Geo& g, int items);
 cudaError_t launch_pair(const Geo& g4, const Geo& go, const PairLaunch& L, const Shape& sh, cudaStream_t s, int* err);
 // dst (geometry g4) <- interior of src (geometry gs), with g4.halo-deep images (FP64, items fields).
 cudaError_t launch_widen(const Geo& g4, void* dst, const Geo& gs, const void* src, int items, const int* item_lo,

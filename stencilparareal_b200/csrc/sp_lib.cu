@@ -150,11 +150,11 @@ struct sp_convection {
         Tune t;
         t.set_all(sh);
         for (int i = 0; i < 4; ++i) t.op[OP_ADJ + i] = default_stage_shape(g[prec], items, true);
-        // FP64 RK4: fused stage pairs, except in the direct kernel's sizes
+        // FP64 RK4: fused stage pairs, except where launches are small
         if (prec == 0 && pair_supported(g4)) {
             t.pair[0] = t.pair[1] = sh.tma ? default_pair_shape(g4, items) : Shape{8, 0, 1};
             t.fused = 1;
-            t.small_direct = sh.tma ? 0 : 1;
+            t.small_stages = !sh.tma || stages_before_pairs(g4, items) ? 1 : 0;
             t.small_cluster = default_cluster_mode(g[0], items);
         }
         return t;
