@@ -98,6 +98,7 @@ struct StageLaunch {
     double c_lam = 0, c_ybar = 0;    // mu_{s-1} = c_lam*lam + c_ybar*ybar_s
     double sigma = 1;                // mu_s = sigma * (stencil input)
     double dnu = 1;                  // d nu / d nu0
+    bool wrap = false;               // wrapping direct kernel: `yin` needs no images, `yout` gets none
     int adj_first = 0;               // 1: lam_acc = lam + ybar (first adjoint stage of a step)
 };
 
@@ -134,6 +135,9 @@ constexpr int kClusterSmemMax = 227 * 1024;
 
 // Launch shape of the single-stage kernels before tuning, for `items` fields per launch.
 Shape default_stage_shape(const Geo& g, int items, bool adjoint = false);
+
+// Whether the (direct) stage kernels of a grid have a wrapping form (StageLaunch::wrap).
+bool wrap_supported(const Geo& g);
 
 // Items with a diffusivity of their own that one launch takes (their weights are
 // kernel arguments, 104 bytes each: within 4 KB); larger batches take several.

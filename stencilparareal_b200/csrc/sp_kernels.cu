@@ -288,22 +288,29 @@ __device__ __forceinline__ void reduce_par(double* g, double* par_acc, double gs
 // Unrolled by two with the next plane prefetched (70-100 registers): 64^3 FP32
 // 11.0, but 128^3 FP64 62.5 and FP32 41.8.
 
-// A chunk by a plain global load.  Not volatile, so that the compiler may move it
-// over the stores of other cells; the addresses come from pointers passed
-// through after_wait, so that it cannot move over griddepcontrol.wait.
+// A chunk by a plain global load, `off` bytes from `base`.  Not volatile, so that the
+// compiler may move it over the stores of other cells; the bases come from pointers
+// passed through after_wait, so that it cannot move over griddepcontrol.wait.
 template <typename T>
-__device__ __forceinline__ Vec<T, V16<T>::N> ldg16(const T* p) {
+__device__ __forceinline__ Vec<T, V16<T>::N> ldg16(const char* base, uint32_t off) {
     Vec<T, V16<T>::N> r;
+    const char* p = base + off;
     if constexpr (sizeof(T) == 8)
         asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.v[0]), "=d"(r.v[1]) : "l"(p));
     else
-        asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]) : "l"(p));
+        asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+            : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3])
+            : "l"(p));
     return r;
 }
 template <typename T>
-__device__ __forceinline__ T* after_wait(T* p) {
+__device__ __forceinline__ Vec<T, V16<T>::N> ldg16(const T* p) {
+    return ldg16<T>(reinterpret_cast<const char*>(p), 0u);
+}
+template <typename T>
+__device__ __forceinline__ const char* after_wait(T* p) {
     asm volatile("" : "+l"(p)::"memory");
-    return p;
+    return reinterpret_cast<const char*>(p);
 }
 
 template <typename T, int OP, int NW>
@@ -325,11 +332,11 @@ __global__ void __launch_bounds__(512)
         const int z1 = min(z0 + a.zchunk, a.nk);
         const long long ob = (long long)b * a.item_stride + a.origin;
         const long long col = ob + (long long)y * a.px + x;
-        const T* S = after_wait(a.yin) + col;
+        const T* S = reinterpret_cast<const T*>(after_wait(a.yin)) + col;
         [[maybe_unused]] const T* pw[3] = {nullptr, nullptr, nullptr};
-        if constexpr (NPW > 0) pw[0] = after_wait(a.pw0) + col;
-        if constexpr (NPW > 1) pw[1] = after_wait(a.pw1) + col;
-        if constexpr (NPW > 2) pw[2] = after_wait(a.pw2) + col;
+        if constexpr (NPW > 0) pw[0] = reinterpret_cast<const T*>(after_wait(a.pw0)) + col;
+        if constexpr (NPW > 1) pw[1] = reinterpret_cast<const T*>(after_wait(a.pw1)) + col;
+        if constexpr (NPW > 2) pw[2] = reinterpret_cast<const T*>(after_wait(a.pw2)) + col;
         const long long pl = a.plane, px = a.px;
         V win[5];  // the column's planes z-2 .. z+2
 #pragma unroll
@@ -375,6 +382,97 @@ __global__ void __launch_bounds__(512)
         }
     }
     if constexpr (OpTraits<OP>::adjoint) reduce_par(g, a.par_acc, a.gs_nu, a.gs_c);
+}
+
+// ---------------------------------------------------------------------------
+// Wrapping direct kernel: the direct kernel for chains of direct stages on grids
+// whose rows are whole chunks.  It takes its neighbours at their wrapped indices,
+// so no stage needs, or writes, periodic images (the driver refreshes those of the
+// field it hands out).  Every offset inside a plane is worked out once per thread,
+// and ZB planes are marched without a loop.
+//
+// What it saves is instructions: a warp's plane of S1 takes 137 (FP64) or 273 (FP32)
+// instead of 211 or 326, a third of which went to images (every warp holds a chunk
+// at an x face, so every warp took that path) and to moving the z-window.  FP32,
+// bound by issue, gains (us per RK4 step: 96^3 18.9 -> 17.4, 128^3 32.2 -> 27.4, 192^3
+// 102 -> 92); FP64 from 100^3 on is bound by what it reads through L2 (100^3 30 ->
+// 27.4, 128^3 51.2 -> 49.0), below by the launches (64^3 12.6 -> 12.1).
+template <typename T, int OP, int NW, int ZB>
+__global__ void __launch_bounds__(512)
+    k_stage_wrap(const __grid_constant__ KArgs<T> a, const __grid_constant__ Weights<T, NW> wt) {
+    constexpr int N = V16<T>::N, ES = (int)sizeof(T), NPW = OpTraits<OP>::npw;
+    constexpr bool RK = OP <= OP_RK_S4;
+    using V = Vec<T, N>;
+    pdl_trigger();
+    pdl_wait();
+    const int b = blockIdx.z;
+    if (a.item_lo && b + a.item_base < *a.item_lo) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = t / a.tiles_x;  // tiles_x: chunks per row
+    const int x = (t - y * a.tiles_x) * N;
+    if (y >= a.nj) return;
+    const int z0 = (a.zrev ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y) * a.zchunk;
+    const int z1 = min(z0 + a.zchunk, a.nk);
+    // byte offsets in a plane of the chunk and its neighbours
+    const uint32_t row = (uint32_t)a.px * ES;
+    const uint32_t o = (uint32_t)y * row + (uint32_t)x * ES;
+    const uint32_t ol = o + (x == 0 ? (uint32_t)(a.ni - N) * ES : (uint32_t)-16);
+    const uint32_t orr = o + (x + N == a.ni ? (uint32_t)(N - a.ni) * ES : 16u);
+    auto wrap_y = [&](int d) { return o + (uint32_t)(d + (y + d < 0 ? a.nj : (y + d >= a.nj ? -a.nj : 0))) * row; };
+    const uint32_t om2 = wrap_y(-2), om1 = wrap_y(-1), op1 = wrap_y(1), op2 = wrap_y(2);
+    const long long pl = a.plane * ES;
+    const long long base = ((long long)b * a.item_stride + a.origin) * ES;
+    const char* F = after_wait(a.yin) + base;
+    auto plane = [&](int z) { return F + (z < 0 ? z + a.nk : (z >= a.nk ? z - a.nk : z)) * pl; };
+    [[maybe_unused]] const char* pw[2] = {nullptr, nullptr};
+    if constexpr (NPW > 0) pw[0] = after_wait(a.pw0) + base;
+    if constexpr (NPW > 1) pw[1] = after_wait(a.pw1) + base;
+    char* Y = reinterpret_cast<char*>(a.yout) + base;
+    [[maybe_unused]] char* A = reinterpret_cast<char*>(a.aout) + base;
+    V win[ZB + 4];  // the column's planes z-2 .. z+ZB+1
+#pragma unroll
+    for (int i = 0; i < 4; ++i) win[i] = ldg16<T>(plane(z0 - 2 + i), o);
+#pragma unroll 1
+    for (int z = z0; z < z1; z += ZB) {
+#pragma unroll
+        for (int i = 0; i < ZB; ++i) win[4 + i] = ldg16<T>(plane(min(z + 2 + i, a.nk + 1)), o);
+#pragma unroll
+        for (int i = 0; i < ZB; ++i) {
+            if (i > 0 && z + i >= z1) break;
+            const long long zo = (z + i) * pl;
+            const char* S = F + zo;
+            const V xl = ldg16<T>(S, ol), xr = ldg16<T>(S, orr);
+            const V ym1 = ldg16<T>(S, om1), yp1 = ldg16<T>(S, op1);
+            const V ym2 = ldg16<T>(S, om2), yp2 = ldg16<T>(S, op2);
+            [[maybe_unused]] V p[2];
+#pragma unroll
+            for (int k = 0; k < NPW; ++k) p[k] = ldg16<T>(pw[k] + zo, o);
+            T row3[3 * N];
+#pragma unroll
+            for (int e = 0; e < N; ++e) { row3[e] = xl.v[e]; row3[N + e] = win[i + 2].v[e]; row3[2 * N + e] = xr.v[e]; }
+            V oy, oa;
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                Nb<T> s;
+                s.c = row3[N + e];
+                s.xm1 = row3[N + e - 1]; s.xp1 = row3[N + e + 1];
+                s.xm2 = row3[N + e - 2]; s.xp2 = row3[N + e + 2];
+                s.ym1 = ym1.v[e]; s.yp1 = yp1.v[e]; s.ym2 = ym2.v[e]; s.yp2 = yp2.v[e];
+                s.zm1 = win[i + 1].v[e]; s.zp1 = win[i + 3].v[e]; s.zm2 = win[i].v[e]; s.zp2 = win[i + 4].v[e];
+                T q0 = 0, q1 = 0, vy = 0, va = 0;
+                if constexpr (NPW > 0) q0 = p[0].v[e];
+                if constexpr (NPW > 1) q1 = p[1].v[e];
+                if constexpr (RK) rk_update<T, OP>(a, rhs_w13(wt.w[NW == 1 ? 0 : b], s), s.c, q0, q1, vy, va);
+                else cell_op<T, OP>(a, s, q0, q1, T(0), vy, va, nullptr, true);
+                oy.v[e] = vy;
+                oa.v[e] = va;
+            }
+            gst16<T>(a.sb_y, reinterpret_cast<T*>(Y + zo + o), oy);
+            if constexpr (OpTraits<OP>::writes_a) gst16<T>(a.sb_a, reinterpret_cast<T*>(A + zo + o), oa);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) win[i] = win[i + ZB];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -708,6 +806,16 @@ cudaError_t launch_direct_T(const Geo& g, const StageLaunch& L, KArgs<T> a, cons
     if (chunks > 0x7fffffffLL || grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
     Weights<T, NW> wt;
     fill_weights(wt, L.coef, L.nu, L.nu_items, L.items);
+    if constexpr (!OpTraits<OP>::adjoint) {
+        if (L.wrap) {
+            switch (std::min(t.zchunk, 4)) {
+                case 1: return launch_pdl(k_stage_wrap<T, OP, NW, 1>, grid, dim3(threads), 0, s, a, wt);
+                case 2: return launch_pdl(k_stage_wrap<T, OP, NW, 2>, grid, dim3(threads), 0, s, a, wt);
+                case 3: return launch_pdl(k_stage_wrap<T, OP, NW, 3>, grid, dim3(threads), 0, s, a, wt);
+                default: return launch_pdl(k_stage_wrap<T, OP, NW, 4>, grid, dim3(threads), 0, s, a, wt);
+            }
+        }
+    }
     return launch_pdl(k_stage_direct<T, OP, NW>, grid, dim3(threads), 0, s, a, wt);
 }
 
@@ -756,6 +864,7 @@ cudaError_t set_attr_op() {
 // NP pointwise slots (prefetch NP-1 planes ahead).
 template <typename T, int OP, int NW>
 cudaError_t launch_op(const Geo& g, const StageLaunch& L, const Shape& t, cudaStream_t s, int* err) {
+    if (L.wrap && (t.tma || !wrap_supported(g))) return cudaErrorInvalidValue;
     const KArgs<T> a = make_args<T>(g, L, t, err);
     if (!t.tma) return launch_direct_T<T, OP, NW>(g, L, a, t, s);
     switch (t.ty) {
@@ -855,9 +964,13 @@ cudaError_t launch_wait_selftest(int* err, unsigned long long limit_ns, cudaStre
 // cells) 58 / 60, 16 of them 126 / 114, one 192^3 175 / 159; FP32 192^3 (7.1M) 102 /
 // 112, 256^3 234 / 204; adjoint (a whole gradient, per step) 96^3 110 / 129, 128^3
 // 251 / 197 -- its direct kernels need 98 registers.  The direct kernel takes as
-// many planes per thread as give one wave of threads (FP64 96^3: 3 planes 23.5, 1
-// or 2 planes 26-27; FP32 95 x 97 x 93: 1 plane 19.9, 2 planes 22.4), at most four
-// (longer chunks gained nothing at 128^3-192^3).
+// many planes per thread as give one wave of threads (FP64 95 x 97 x 93: 3 planes
+// 24.0, 2 planes 26.7; FP32 1 plane 19.9, 2 planes 22.4), at most four (longer
+// chunks gained nothing at 128^3-192^3); its wrapping form two planes beyond one
+// wave (FP64 100^3: 1, 2, 3, 4 planes 28.9, 27.4, 31.5, 32.5; 128^3 54.7, 49.0, 49.8,
+// 52.7; FP32 128^3 29, 27.4, 28.7, 31).
+bool wrap_supported(const Geo& g) { return g.ni % (16 / g.es) == 0 && g.plane * g.es <= 0xffffffffLL; }
+
 Shape default_stage_shape(const Geo& g, int items, bool adjoint) {
     const long long direct = adjoint ? 1'500'000 : (g.es == 8 ? 3'000'000 : 12'000'000);
     const long long cells = (long long)g.ni * g.nj * g.nk * items;
@@ -867,8 +980,9 @@ Shape default_stage_shape(const Geo& g, int items, bool adjoint) {
         const long long threads = (long long)((g.ni + n - 1) / n) * g.nj * g.nk * items;
         const long long wave = 148LL * (g.es == 8 ? 1024 : 1792);
         sh.tma = 0;
-        sh.ty = g.es == 8 ? 8 : 4;
-        sh.zchunk = (int)std::min(4LL, (threads + wave - 1) / wave);
+        const bool wrap = !adjoint && wrap_supported(g);
+        sh.ty = g.es == 8 && !wrap ? 8 : 4;
+        sh.zchunk = (int)std::min(wrap ? 2LL : 4LL, (threads + wave - 1) / wave);
         return sh;
     }
     // TMA rings: 4-row tiles, z-chunks that give at least ~8 CTAs per SM

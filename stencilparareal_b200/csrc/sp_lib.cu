@@ -206,6 +206,14 @@ struct NuSrc {
     const double* items = nullptr;
 };
 
+// Whether a tune's RK4 (or Euler) steps run as a chain of wrapping direct kernels:
+// they read no periodic images and write none.
+bool wraps(const Geo& g, const Tune& t, bool rk) {
+    if (!wrap_supported(g)) return false;
+    if (!rk) return !t.op[OP_EULER].tma;
+    return !t.op[OP_RK_S1].tma && !t.op[OP_RK_S2].tma && !t.op[OP_RK_S3].tma && !t.op[OP_RK_S4].tma;
+}
+
 // One RK4 step over `items` fields: in -> out, with scratch ya/yb/acc.
 cudaError_t enqueue_rk4_step3(const Geo& g, int prec, const Coef& c, double dt, NuSrc nu, const void* in, void* out,
                               void* ya, void* yb, void* yc, void* acc, int items, const int* item_lo, int item_base,
@@ -218,6 +226,7 @@ cudaError_t enqueue_rk4_step3(const Geo& g, int prec, const Coef& c, double dt, 
     L.nu = nu.nu;
     L.nu_items = nu.items;
     L.coef = c;
+    L.wrap = wraps(g, t, true);
     const double dthalf = dt * .5;  // Convection.cpp:320
     // S1
     L.op = OP_RK_S1; L.yin = in; L.yout = ya; L.acc = acc; L.c_y = dthalf; L.c_acc = dt / 6.;
@@ -252,6 +261,7 @@ cudaError_t enqueue_euler_step(const Geo& g, int prec, const Coef& c, double dt,
     L.nu = nu.nu;
     L.nu_items = nu.items;
     L.coef = c;
+    L.wrap = wraps(g, t, false);
     L.yin = in;
     L.yout = out;
     L.c_y = dt;
@@ -487,6 +497,8 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
             SP_CUDA(cudaMemcpyAsync(out, src, g.total * g.es, cudaMemcpyDeviceToDevice, s));
         }
     }
+    if (!resident && !(rk && prec == 0 && t.pairs() && pair_supported(h->g4)) && wraps(g, t, rk))
+        SP_CUDA(launch_periodicity(g, out, 1, s));  // the wrapping kernels wrote no images
     return SP_OK;
 }
 
@@ -930,6 +942,7 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
                     Shape sh;
                     sh.tma = kind; sh.ty = ty; sh.zchunk = zc;
                     t.set_all(sh);
+                    L.wrap = kind == 0 && wrap_supported(g);  // as in a step of direct kernels
                     cudaError_t e = launch_stage(g, L, t, s, h->err.as<int>());
                     if (e != cudaSuccess) { cudaGetLastError(); continue; }
                     float ms = 1e30f;
