@@ -121,7 +121,7 @@ struct sp_convection {
     DevBuf err;         // device error word
     DevBuf red;         // reduction scratch (8 doubles)
     DevBuf dense;       // staging for the host-buffer entry point
-    DevBuf adj_ckpt, adj_seg, adj_work, adj_par;  // adjoint workspace, kept between calls
+    DevBuf adj;         // adjoint workspace, kept between calls
     std::map<std::tuple<int, int>, Tune> tunes;     // (prec, items) -> tune
     std::map<std::tuple<int, int>, Tune> defaults;  // the same, before tuning
     std::map<std::tuple<int, const void*, double, double, int>, GraphEntry> graphs;
@@ -532,9 +532,11 @@ int sp_convection_create(const sp_params* p, int device, sp_convection** out) {
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(SP_ERR_UNSUPPORTED, "no CUDA device");
     if (device < 0 || device >= ndev) return fail(SP_ERR_INVALID, "device %d out of range", device);
     SP_CUDA(cudaSetDevice(device));
-    cudaDeviceProp prop;
-    SP_CUDA(cudaGetDeviceProperties(&prop, device));
-    if (prop.major < 10) return fail(SP_ERR_UNSUPPORTED, "this library is built for sm_100a (found sm_%d%d)", prop.major, prop.minor);
+    // two attributes, not cudaGetDeviceProperties: that took 2.5 of the 2.9 ms a handle took
+    int major = 0, minor = 0;
+    SP_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    SP_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    if (major < 10) return fail(SP_ERR_UNSUPPORTED, "this library is built for sm_100a (found sm_%d%d)", major, minor);
     std::unique_ptr<sp_convection> h(new sp_convection());
     h->P = *p;
     h->device = device;
@@ -1922,18 +1924,16 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
     const int nseg = n > 0 ? (n + ck - 1) / ck : 0;
     const Geo& g = h->g[0];
     const size_t fb = (size_t)g.total * 8;
-    if ((rc = h->ensure_scratch(0, 1))) return rc;
-    DevBuf& ckpt = h->adj_ckpt;
-    DevBuf& seg = h->adj_seg;
-    DevBuf& work = h->adj_work;
-    DevBuf& par = h->adj_par;
-    // work: qn, lam, lam_acc, mu_a, mu_b, dummy
-    if (ckpt.alloc(std::max(nseg, 1) * fb) != cudaSuccess || seg.alloc((size_t)4 * ck * fb) != cudaSuccess ||
-        work.alloc(6 * fb) != cudaSuccess || par.alloc(8 * sizeof(double)) != cudaSuccess)
+    // One allocation (each costs ~0.35 ms, and as much again to free): nseg checkpoints,
+    // [y2 | y3 | y4 | state] for the ck steps of a segment, nine work fields (qn, lam,
+    // lam_acc, mu_a, mu_b, a field for results nobody reads, RK4 scratch), eight sums
+    const size_t nfield = (size_t)std::max(nseg, 1) + 4 * (size_t)ck + 9;
+    if (h->adj.alloc(nfield * fb + 8 * sizeof(double)) != cudaSuccess)
         return fail(SP_ERR_NOMEM, "adjoint buffers (%d checkpoints, %d-step segments)", nseg, ck);
-    auto CK = [&](int i) { return ckpt.as<double>() + (size_t)i * g.total; };
-    auto SG = [&](int i) { return seg.as<double>() + (size_t)i * g.total; };  // [y2 | y3 | y4 | state] x ck
-    auto WK = [&](int i) { return work.as<double>() + (size_t)i * g.total; };
+    double* const par = h->adj.as<double>() + nfield * g.total;
+    auto CK = [&](int i) { return h->adj.as<double>() + (size_t)i * g.total; };
+    auto SG = [&](int i) { return CK(std::max(nseg, 1)) + (size_t)i * g.total; };
+    auto WK = [&](int i) { return SG(4 * ck) + (size_t)i * g.total; };
     double* qn = WK(0);
     double* lam = WK(1);
     double* lamacc = WK(2);
@@ -1942,11 +1942,11 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
     double* dummy = WK(5);
     const Tune t = h->tune(0, 1);
     int* err = h->err.as<int>();
-    double* ya = static_cast<double*>(h->sbuf(0, 0, 1));
-    double* yb = static_cast<double*>(h->sbuf(0, 1, 1));
-    double* acc = static_cast<double*>(h->sbuf(0, 2, 1));
+    double* ya = WK(6);
+    double* yb = WK(7);
+    double* acc = WK(8);
     const double nu0 = h->P.nu0, nuf = h->P.nufreq;
-    SP_CUDA(cudaMemsetAsync(par.p, 0, 8 * sizeof(double), s));
+    SP_CUDA(cudaMemsetAsync(par, 0, 8 * sizeof(double), s));
     // forward sweep, keeping checkpoints
     SP_CUDA(cudaMemcpyAsync(nseg > 0 ? CK(0) : qn, q0, fb, cudaMemcpyDeviceToDevice, s));
     SP_CUDA(launch_periodicity(g, nseg > 0 ? CK(0) : qn, 1, s));
@@ -1965,7 +1965,7 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
         SP_CUDA(cudaMemcpyAsync(lam, lambda_n, fb, cudaMemcpyDeviceToDevice, s));
         SP_CUDA(launch_periodicity(g, lam, 1, s));
     } else {
-        SP_CUDA(launch_misfit(g, qn, q_target, lam, par.as<double>() + 4, s));
+        SP_CUDA(launch_misfit(g, qn, q_target, lam, par + 4, s));
     }
     // backward sweep
     for (int sg = nseg - 1; sg >= 0; --sg) {
@@ -1988,7 +1988,7 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
             L.coef = h->coef;
             L.nu = computenu(nu0, nuf, tt);
             L.dnu = 1. + .5 * std::sin(nuf * tt);
-            L.par_acc = par.as<double>();
+            L.par_acc = par;
             // A4: stencil lam (mu4 = h/6 lam)
             L.op = OP_ADJ + 0; L.yin = lam; L.sigma = dt / 6.; L.ypt = Y4(i);
             L.yout = mua; L.lam_acc = lamacc; L.c_ybar = dt; L.c_lam = dt / 3.;
@@ -2009,7 +2009,7 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
     }
     SP_CUDA(cudaMemcpyAsync(grad_q0, lam, fb, cudaMemcpyDeviceToDevice, s));
     double hp[8];
-    SP_CUDA(cudaMemcpyAsync(hp, par.p, sizeof hp, cudaMemcpyDeviceToHost, s));
+    SP_CUDA(cudaMemcpyAsync(hp, par, sizeof hp, cudaMemcpyDeviceToHost, s));
     if ((rc = sp_convection_synchronize(h))) return rc;
     if (grad_par) for (int i = 0; i < 4; ++i) grad_par[i] = hp[i];
     if (J) *J = lambda_n ? 0. : hp[4];
