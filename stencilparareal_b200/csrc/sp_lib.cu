@@ -238,7 +238,8 @@ cudaError_t enqueue_rk4_step3(const Geo& g, int prec, const Coef& c, double dt, 
     // S3
     L.op = OP_RK_S3; L.yin = yb; L.q = in; L.yout = yc; L.c_y = dt; L.c_acc = dt / 3.;
     if ((e = launch_stage(g, L, t, s, err)) != cudaSuccess) return e;
-    // S4
+    // S4 (not when only the stage values are wanted)
+    if (!out) return cudaSuccess;
     L.op = OP_RK_S4; L.yin = yc; L.q = in; L.yout = out; L.c_acc = dt / 6.;
     return launch_stage(g, L, t, s, err);
 }
@@ -1925,9 +1926,9 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
     const Geo& g = h->g[0];
     const size_t fb = (size_t)g.total * 8;
     // One allocation (each costs ~0.35 ms, and as much again to free): nseg checkpoints,
-    // [y2 | y3 | y4 | state] for the ck steps of a segment, nine work fields (qn, lam,
-    // lam_acc, mu_a, mu_b, a field for results nobody reads, RK4 scratch), eight sums
-    const size_t nfield = (size_t)std::max(nseg, 1) + 4 * (size_t)ck + 9;
+    // [y2 | y3 | y4 | state] for the ck steps of a segment, eight work fields (qn, lam,
+    // lam_acc, mu_a, mu_b, RK4 scratch), eight sums
+    const size_t nfield = (size_t)std::max(nseg, 1) + 4 * (size_t)ck + 8;
     if (h->adj.alloc(nfield * fb + 8 * sizeof(double)) != cudaSuccess)
         return fail(SP_ERR_NOMEM, "adjoint buffers (%d checkpoints, %d-step segments)", nseg, ck);
     double* const par = h->adj.as<double>() + nfield * g.total;
@@ -1939,20 +1940,35 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
     double* lamacc = WK(2);
     double* mua = WK(3);
     double* mub = WK(4);
-    double* dummy = WK(5);
     const Tune t = h->tune(0, 1);
     int* err = h->err.as<int>();
-    double* ya = WK(6);
-    double* yb = WK(7);
-    double* acc = WK(8);
+    double* ya = WK(5);
+    double* yb = WK(6);
+    double* acc = WK(7);
     const double nu0 = h->P.nu0, nuf = h->P.nufreq;
     SP_CUDA(cudaMemsetAsync(par, 0, 8 * sizeof(double), s));
-    // forward sweep, keeping checkpoints
+    auto Y2 = [&](int i) { return SG(4 * i + 0); };
+    auto Y3 = [&](int i) { return SG(4 * i + 1); };
+    auto Y4 = [&](int i) { return SG(4 * i + 2); };
+    // the steps of segment sg with their stage inputs kept; the state after the last one goes to `end`
+    auto stages_of_segment = [&](int sg, double* end) -> int {
+        const int s0 = sg * ck, m = std::min(n, s0 + ck) - s0;
+        for (int i = 0; i < m; ++i) {
+            const double tt = tStart + (s0 + i) * dt;
+            const double* st = i == 0 ? CK(sg) : SG(4 * (i - 1) + 3);
+            SP_CUDA(enqueue_rk4_step3(g, 0, h->coef, dt, NuSrc{computenu(nu0, nuf, tt), nullptr}, st,
+                                      i + 1 < m ? SG(4 * i + 3) : end, Y2(i), Y3(i), Y4(i), acc, 1, nullptr, 0, t, s,
+                                      err));
+        }
+        return SP_OK;
+    };
+    // forward sweep, keeping checkpoints and the stage inputs of the last segment,
+    // with which the backward sweep starts (that segment is not recomputed)
     SP_CUDA(cudaMemcpyAsync(nseg > 0 ? CK(0) : qn, q0, fb, cudaMemcpyDeviceToDevice, s));
     SP_CUDA(launch_periodicity(g, nseg > 0 ? CK(0) : qn, 1, s));
-    for (int sg = 0; sg < nseg; ++sg) {
-        const int s0 = sg * ck, s1 = std::min(n, s0 + ck);
-        double* dst = (sg + 1 < nseg) ? CK(sg + 1) : qn;
+    for (int sg = 0; sg + 1 < nseg; ++sg) {
+        const int s0 = sg * ck, s1 = s0 + ck;
+        double* dst = CK(sg + 1);
         for (int st = s0; st < s1; ++st) {
             const double tt = tStart + st * dt;
             SP_CUDA(enqueue_rk4_step(g, 0, h->coef, dt, NuSrc{computenu(nu0, nuf, tt), nullptr},
@@ -1960,6 +1976,7 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
                                      0, t, s, err));
         }
     }
+    if (nseg > 0 && (rc = stages_of_segment(nseg - 1, qn))) return rc;
     // terminal adjoint
     if (lambda_n) {
         SP_CUDA(cudaMemcpyAsync(lam, lambda_n, fb, cudaMemcpyDeviceToDevice, s));
@@ -1969,17 +1986,9 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
     }
     // backward sweep
     for (int sg = nseg - 1; sg >= 0; --sg) {
-        const int s0 = sg * ck, s1 = std::min(n, s0 + ck), m = s1 - s0;
-        auto Y2 = [&](int i) { return SG(4 * i + 0); };
-        auto Y3 = [&](int i) { return SG(4 * i + 1); };
-        auto Y4 = [&](int i) { return SG(4 * i + 2); };
+        const int s0 = sg * ck, m = std::min(n, s0 + ck) - s0;
         auto ST = [&](int i) { return i == 0 ? CK(sg) : SG(4 * (i - 1) + 3); };  // state at step s0+i
-        for (int i = 0; i < m; ++i) {
-            const double tt = tStart + (s0 + i) * dt;
-            double* next = (i + 1 < m) ? SG(4 * i + 3) : dummy;
-            SP_CUDA(enqueue_rk4_step3(g, 0, h->coef, dt, NuSrc{computenu(nu0, nuf, tt), nullptr}, ST(i), next, Y2(i),
-                                      Y3(i), Y4(i), acc, 1, nullptr, 0, t, s, err));
-        }
+        if (sg + 1 < nseg && (rc = stages_of_segment(sg, nullptr))) return rc;
         for (int i = m - 1; i >= 0; --i) {
             const double tt = tStart + (s0 + i) * dt;
             StageLaunch L;
