@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(512)
 // instead of 211 or 326, a third of which went to images (every warp holds a chunk
 // at an x face, so every warp took that path) and to moving the z-window.  FP32,
 // bound by issue, gains (us per RK4 step: 96^3 18.9 -> 17.4, 128^3 32.2 -> 27.4, 192^3
-// 102 -> 92); FP64 from 100^3 on is bound by what it reads through L2 (100^3 30 ->
+// 102 -> 92; a gradient, in FP64, 64^3 58 -> 49, 96^3 110 -> 90); FP64 from 100^3 on is bound by what it reads through L2 (100^3 30 ->
 // 27.4, 128^3 51.2 -> 49.0), below by the launches (64^3 12.6 -> 12.1).
 template <typename T, int OP, int NW, int ZB>
 __global__ void __launch_bounds__(512)
@@ -410,69 +410,75 @@ __global__ void __launch_bounds__(512)
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = t / a.tiles_x;  // tiles_x: chunks per row
     const int x = (t - y * a.tiles_x) * N;
-    if (y >= a.nj) return;
-    const int z0 = (a.zrev ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y) * a.zchunk;
-    const int z1 = min(z0 + a.zchunk, a.nk);
-    // byte offsets in a plane of the chunk and its neighbours
-    const uint32_t row = (uint32_t)a.px * ES;
-    const uint32_t o = (uint32_t)y * row + (uint32_t)x * ES;
-    const uint32_t ol = o + (x == 0 ? (uint32_t)(a.ni - N) * ES : (uint32_t)-16);
-    const uint32_t orr = o + (x + N == a.ni ? (uint32_t)(N - a.ni) * ES : 16u);
-    auto wrap_y = [&](int d) { return o + (uint32_t)(d + (y + d < 0 ? a.nj : (y + d >= a.nj ? -a.nj : 0))) * row; };
-    const uint32_t om2 = wrap_y(-2), om1 = wrap_y(-1), op1 = wrap_y(1), op2 = wrap_y(2);
-    const long long pl = a.plane * ES;
-    const long long base = ((long long)b * a.item_stride + a.origin) * ES;
-    const char* F = after_wait(a.yin) + base;
-    auto plane = [&](int z) { return F + (z < 0 ? z + a.nk : (z >= a.nk ? z - a.nk : z)) * pl; };
-    [[maybe_unused]] const char* pw[2] = {nullptr, nullptr};
-    if constexpr (NPW > 0) pw[0] = after_wait(a.pw0) + base;
-    if constexpr (NPW > 1) pw[1] = after_wait(a.pw1) + base;
-    char* Y = reinterpret_cast<char*>(a.yout) + base;
-    [[maybe_unused]] char* A = reinterpret_cast<char*>(a.aout) + base;
-    V win[ZB + 4];  // the column's planes z-2 .. z+ZB+1
+    [[maybe_unused]] double g[4] = {0., 0., 0., 0.};
+    auto march = [&]() {
+        const int z0 = (a.zrev ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y) * a.zchunk;
+        const int z1 = min(z0 + a.zchunk, a.nk);
+        // byte offsets in a plane of the chunk and its neighbours
+        const uint32_t row = (uint32_t)a.px * ES;
+        const uint32_t o = (uint32_t)y * row + (uint32_t)x * ES;
+        const uint32_t ol = o + (x == 0 ? (uint32_t)(a.ni - N) * ES : (uint32_t)-16);
+        const uint32_t orr = o + (x + N == a.ni ? (uint32_t)(N - a.ni) * ES : 16u);
+        auto wrap_y = [&](int d) { return o + (uint32_t)(d + (y + d < 0 ? a.nj : (y + d >= a.nj ? -a.nj : 0))) * row; };
+        const uint32_t om2 = wrap_y(-2), om1 = wrap_y(-1), op1 = wrap_y(1), op2 = wrap_y(2);
+        const long long pl = a.plane * ES;
+        const long long base = ((long long)b * a.item_stride + a.origin) * ES;
+        const char* F = after_wait(a.yin) + base;
+        auto plane = [&](int z) { return F + (z < 0 ? z + a.nk : (z >= a.nk ? z - a.nk : z)) * pl; };
+        [[maybe_unused]] const char* pw[3] = {nullptr, nullptr, nullptr};
+        if constexpr (NPW > 0) pw[0] = after_wait(a.pw0) + base;
+        if constexpr (NPW > 1) pw[1] = after_wait(a.pw1) + base;
+        if constexpr (NPW > 2) pw[2] = after_wait(a.pw2) + base;
+        char* Y = reinterpret_cast<char*>(a.yout) + base;
+        [[maybe_unused]] char* A = reinterpret_cast<char*>(a.aout) + base;
+        V win[ZB + 4];  // the column's planes z-2 .. z+ZB+1
 #pragma unroll
-    for (int i = 0; i < 4; ++i) win[i] = ldg16<T>(plane(z0 - 2 + i), o);
+        for (int i = 0; i < 4; ++i) win[i] = ldg16<T>(plane(z0 - 2 + i), o);
 #pragma unroll 1
-    for (int z = z0; z < z1; z += ZB) {
+        for (int z = z0; z < z1; z += ZB) {
 #pragma unroll
-        for (int i = 0; i < ZB; ++i) win[4 + i] = ldg16<T>(plane(min(z + 2 + i, a.nk + 1)), o);
+            for (int i = 0; i < ZB; ++i) win[4 + i] = ldg16<T>(plane(min(z + 2 + i, a.nk + 1)), o);
 #pragma unroll
-        for (int i = 0; i < ZB; ++i) {
-            if (i > 0 && z + i >= z1) break;
-            const long long zo = (z + i) * pl;
-            const char* S = F + zo;
-            const V xl = ldg16<T>(S, ol), xr = ldg16<T>(S, orr);
-            const V ym1 = ldg16<T>(S, om1), yp1 = ldg16<T>(S, op1);
-            const V ym2 = ldg16<T>(S, om2), yp2 = ldg16<T>(S, op2);
-            [[maybe_unused]] V p[2];
+            for (int i = 0; i < ZB; ++i) {
+                if (i > 0 && z + i >= z1) break;
+                const long long zo = (z + i) * pl;
+                const char* S = F + zo;
+                const V xl = ldg16<T>(S, ol), xr = ldg16<T>(S, orr);
+                const V ym1 = ldg16<T>(S, om1), yp1 = ldg16<T>(S, op1);
+                const V ym2 = ldg16<T>(S, om2), yp2 = ldg16<T>(S, op2);
+                [[maybe_unused]] V p[3];
 #pragma unroll
-            for (int k = 0; k < NPW; ++k) p[k] = ldg16<T>(pw[k] + zo, o);
-            T row3[3 * N];
+                for (int k = 0; k < NPW; ++k) p[k] = ldg16<T>(pw[k] + zo, o);
+                T row3[3 * N];
 #pragma unroll
-            for (int e = 0; e < N; ++e) { row3[e] = xl.v[e]; row3[N + e] = win[i + 2].v[e]; row3[2 * N + e] = xr.v[e]; }
-            V oy, oa;
+                for (int e = 0; e < N; ++e) { row3[e] = xl.v[e]; row3[N + e] = win[i + 2].v[e]; row3[2 * N + e] = xr.v[e]; }
+                V oy, oa;
 #pragma unroll
-            for (int e = 0; e < N; ++e) {
-                Nb<T> s;
-                s.c = row3[N + e];
-                s.xm1 = row3[N + e - 1]; s.xp1 = row3[N + e + 1];
-                s.xm2 = row3[N + e - 2]; s.xp2 = row3[N + e + 2];
-                s.ym1 = ym1.v[e]; s.yp1 = yp1.v[e]; s.ym2 = ym2.v[e]; s.yp2 = yp2.v[e];
-                s.zm1 = win[i + 1].v[e]; s.zp1 = win[i + 3].v[e]; s.zm2 = win[i].v[e]; s.zp2 = win[i + 4].v[e];
-                T q0 = 0, q1 = 0, vy = 0, va = 0;
-                if constexpr (NPW > 0) q0 = p[0].v[e];
-                if constexpr (NPW > 1) q1 = p[1].v[e];
-                if constexpr (RK) rk_update<T, OP>(a, rhs_w13(wt.w[NW == 1 ? 0 : b], s), s.c, q0, q1, vy, va);
-                else cell_op<T, OP>(a, s, q0, q1, T(0), vy, va, nullptr, true);
-                oy.v[e] = vy;
-                oa.v[e] = va;
+                for (int e = 0; e < N; ++e) {
+                    Nb<T> s;
+                    s.c = row3[N + e];
+                    s.xm1 = row3[N + e - 1]; s.xp1 = row3[N + e + 1];
+                    s.xm2 = row3[N + e - 2]; s.xp2 = row3[N + e + 2];
+                    s.ym1 = ym1.v[e]; s.yp1 = yp1.v[e]; s.ym2 = ym2.v[e]; s.yp2 = yp2.v[e];
+                    s.zm1 = win[i + 1].v[e]; s.zp1 = win[i + 3].v[e]; s.zm2 = win[i].v[e]; s.zp2 = win[i + 4].v[e];
+                    T q0 = 0, q1 = 0, q2 = 0, vy = 0, va = 0;
+                    if constexpr (NPW > 0) q0 = p[0].v[e];
+                    if constexpr (NPW > 1) q1 = p[1].v[e];
+                    if constexpr (NPW > 2) q2 = p[2].v[e];
+                    if constexpr (RK) rk_update<T, OP>(a, rhs_w13(wt.w[NW == 1 ? 0 : b], s), s.c, q0, q1, vy, va);
+                    else cell_op<T, OP>(a, s, q0, q1, q2, vy, va, g, true);
+                    oy.v[e] = vy;
+                    oa.v[e] = va;
+                }
+                gst16<T>(a.sb_y, reinterpret_cast<T*>(Y + zo + o), oy);
+                if constexpr (OpTraits<OP>::writes_a) gst16<T>(a.sb_a, reinterpret_cast<T*>(A + zo + o), oa);
             }
-            gst16<T>(a.sb_y, reinterpret_cast<T*>(Y + zo + o), oy);
-            if constexpr (OpTraits<OP>::writes_a) gst16<T>(a.sb_a, reinterpret_cast<T*>(A + zo + o), oa);
-        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) win[i] = win[i + ZB];
-    }
+            for (int i = 0; i < 4; ++i) win[i] = win[i + ZB];
+        }
+    };
+    if (y < a.nj) march();
+    if constexpr (OpTraits<OP>::adjoint) reduce_par(g, a.par_acc, a.gs_nu, a.gs_c);
 }
 
 // ---------------------------------------------------------------------------
@@ -806,14 +812,13 @@ cudaError_t launch_direct_T(const Geo& g, const StageLaunch& L, KArgs<T> a, cons
     if (chunks > 0x7fffffffLL || grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
     Weights<T, NW> wt;
     fill_weights(wt, L.coef, L.nu, L.nu_items, L.items);
-    if constexpr (!OpTraits<OP>::adjoint) {
-        if (L.wrap) {
-            switch (std::min(t.zchunk, 4)) {
-                case 1: return launch_pdl(k_stage_wrap<T, OP, NW, 1>, grid, dim3(threads), 0, s, a, wt);
-                case 2: return launch_pdl(k_stage_wrap<T, OP, NW, 2>, grid, dim3(threads), 0, s, a, wt);
-                case 3: return launch_pdl(k_stage_wrap<T, OP, NW, 3>, grid, dim3(threads), 0, s, a, wt);
-                default: return launch_pdl(k_stage_wrap<T, OP, NW, 4>, grid, dim3(threads), 0, s, a, wt);
-            }
+    if (L.wrap) {
+        constexpr int ZMAX = OpTraits<OP>::adjoint ? 2 : 4;  // (adjoint stages: 100 registers with two planes)
+        switch (std::min(t.zchunk, ZMAX)) {
+            case 1: return launch_pdl(k_stage_wrap<T, OP, NW, 1>, grid, dim3(threads), 0, s, a, wt);
+            case 2: return launch_pdl(k_stage_wrap<T, OP, NW, 2>, grid, dim3(threads), 0, s, a, wt);
+            case 3: return launch_pdl(k_stage_wrap<T, OP, NW, std::min(3, ZMAX)>, grid, dim3(threads), 0, s, a, wt);
+            default: return launch_pdl(k_stage_wrap<T, OP, NW, ZMAX>, grid, dim3(threads), 0, s, a, wt);
         }
     }
     return launch_pdl(k_stage_direct<T, OP, NW>, grid, dim3(threads), 0, s, a, wt);
@@ -962,8 +967,8 @@ cudaError_t launch_wait_selftest(int* err, unsigned long long limit_ns, cudaStre
 // The direct kernel up to a number of cells per launch, the TMA rings beyond.
 // Where the lines lie (us per RK4 step, direct / TMA): FP64 8 fields of 64^3 (2.1M
 // cells) 58 / 60, 16 of them 126 / 114, one 192^3 175 / 159; FP32 192^3 (7.1M) 102 /
-// 112, 256^3 234 / 204; adjoint (a whole gradient, per step) 96^3 110 / 129, 128^3
-// 251 / 197 -- its direct kernels need 98 registers.  The direct kernel takes as
+// 112, 256^3 234 / 204; adjoint (a whole gradient, per step) 96^3 90 / 115, 128^3
+// 193 / 177.  The direct kernel takes as
 // many planes per thread as give one wave of threads (FP64 95 x 97 x 93: 3 planes
 // 24.0, 2 planes 26.7; FP32 1 plane 19.9, 2 planes 22.4), at most four (longer
 // chunks gained nothing at 128^3-192^3); its wrapping form two planes beyond one
@@ -980,7 +985,7 @@ Shape default_stage_shape(const Geo& g, int items, bool adjoint) {
         const long long threads = (long long)((g.ni + n - 1) / n) * g.nj * g.nk * items;
         const long long wave = 148LL * (g.es == 8 ? 1024 : 1792);
         sh.tma = 0;
-        const bool wrap = !adjoint && wrap_supported(g);
+        const bool wrap = wrap_supported(g);
         sh.ty = g.es == 8 && !wrap ? 8 : 4;
         sh.zchunk = (int)std::min(wrap ? 2LL : 4LL, (threads + wave - 1) / wave);
         return sh;

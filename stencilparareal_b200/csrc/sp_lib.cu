@@ -214,6 +214,11 @@ bool wraps(const Geo& g, const Tune& t, bool rk) {
     return !t.op[OP_RK_S1].tma && !t.op[OP_RK_S2].tma && !t.op[OP_RK_S3].tma && !t.op[OP_RK_S4].tma;
 }
 
+bool wraps_adjoint(const Geo& g, const Tune& t) {
+    return wrap_supported(g) && !t.op[OP_ADJ].tma && !t.op[OP_ADJ + 1].tma && !t.op[OP_ADJ + 2].tma &&
+           !t.op[OP_ADJ + 3].tma;
+}
+
 // One RK4 step over `items` fields: in -> out, with scratch ya/yb/acc.
 cudaError_t enqueue_rk4_step3(const Geo& g, int prec, const Coef& c, double dt, NuSrc nu, const void* in, void* out,
                               void* ya, void* yb, void* yc, void* acc, int items, const int* item_lo, int item_base,
@@ -1997,6 +2002,7 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
             L.coef = h->coef;
             L.nu = computenu(nu0, nuf, tt);
             L.dnu = 1. + .5 * std::sin(nuf * tt);
+            L.wrap = wraps_adjoint(g, t);
             L.par_acc = par;
             // A4: stencil lam (mu4 = h/6 lam)
             L.op = OP_ADJ + 0; L.yin = lam; L.sigma = dt / 6.; L.ypt = Y4(i);
@@ -2017,6 +2023,7 @@ extern "C" int sp_adjoint_rk4(sp_convection* h, const double* q0, const double* 
         }
     }
     SP_CUDA(cudaMemcpyAsync(grad_q0, lam, fb, cudaMemcpyDeviceToDevice, s));
+    if (wraps_adjoint(g, t)) SP_CUDA(launch_periodicity(g, grad_q0, 1, s));  // those kernels wrote no images
     double hp[8];
     SP_CUDA(cudaMemcpyAsync(hp, par, sizeof hp, cudaMemcpyDeviceToHost, s));
     if ((rc = sp_convection_synchronize(h))) return rc;

@@ -94,3 +94,23 @@ def test_parareal_with_one_diffusivity_per_slice(sp, orc, slices):
     p = orc.params(n, dx=1.0 / 18, nu0=0.02, nufreq=40.0, cx=1.0, cy=-0.5, cz=0.25)
     cfg = orc.parareal_cfg(1e-4 * total, slices, total, 2 * slices, 2)
     assert rel_l2(got[0], orc.parareal(p, cfg, q0)[0]) < 1e-11
+
+
+@pytest.mark.parametrize("n", [(32, 12, 10), (18, 7, 5), (17, 9, 6), (2, 3, 5)])
+def test_adjoint_direct_equals_tma(sp, n):
+    """Gradient fields of the direct adjoint stages (wrapping on even widths) and the TMA ring."""
+    from stencilparareal_b200.adjoint import misfit_gradient
+    c = conv_of(sp, n)
+    q0, qt = c.field(), c.field()
+    c.upload(q0, gaussian_noise(*n, seed=8))
+    c.upload(qt, gaussian_noise(*n, seed=9))
+    want = None
+    for tune in [(4, 8, 1), (8, 1, 0), (4, 2, 0), (16, 5, 0)]:
+        c.set_tune(sp.SP_F64, 1, *tune)
+        J, grad, gp = misfit_gradient(c, q0, qt, 0.0, 1e-4, 7, checkpoint_every=3)
+        got = c.download(grad)
+        if want is None:
+            want, par = got, gp
+        assert np.array_equal(got, want), tune
+        assert np.allclose(gp, par, rtol=1e-9, atol=0), tune
+        assert halo_ok(c, grad), tune
