@@ -1346,10 +1346,10 @@ struct sp_parareal {
 namespace {
 
 // Coarse propagation G of one field: src (FP64 slice input, geometry g64) ->
-// result in pr->gt(pr->coarse_res), n steps from t0.  Every kernel is gated by
-// item_lo against `item` when gate is set.
+// result in pr->gt(pr->coarse_res), n steps, the first..first+n-1 of a run from t0.
+// Every kernel is gated by item_lo against `item` when gate is set.
 int enqueue_coarse(sp_parareal* pr, const void* src, const Geo& gsrc, double t0, int n, bool gate, int item,
-                   cudaStream_t s) {
+                   cudaStream_t s, int first = 0) {
     sp_convection* h = pr->prop;
     const int cp = pr->cprec;
     const Geo& gc = pr->gc;
@@ -1366,7 +1366,7 @@ int enqueue_coarse(sp_parareal* pr, const void* src, const Geo& gsrc, double t0,
     void* cur = A;
     void* other = B;
     for (int i = 0; i < n; ++i) {
-        const double tt = i == 0 ? t0 : t0 + i * pr->dtC;
+        const double tt = first + i == 0 ? t0 : t0 + (first + i) * pr->dtC;
         const NuSrc nu{computenu(h->P.nu0, h->P.nufreq, tt), nullptr};
         if (pr->cfg.coarse_scheme == SP_COARSE_RK4) {
             SP_CUDA(enqueue_rk4_step(gc, cp, h->coef, pr->dtC, nu, cur, cur, ya, yb, acc, 1, lo, item, t, s, err));
@@ -1665,8 +1665,11 @@ int enqueue_predictor(sp_parareal* pr, const double* initial, cudaStream_t s) {
             SP_CUDA(launch_convert(g, pr->u(r + 1), pr->gc, pr->gt(pr->coarse_res), s));
         }
     } else {
+        // nu(t) varies: the run from t=0 goes on from the slice before, step for
+        // step at the times of one run (the detour through FP64 changes no value):
+        // tsC steps per slice, not tsC*r (16 slices of 64^3 x 8 steps: 3.9 -> 1.3 ms)
         for (int r = 1; r < P; ++r) {
-            if ((rc = enqueue_coarse(pr, initial, g, 0., pr->tsC * (F0 + r), false, 0, s))) return rc;
+            if ((rc = enqueue_coarse(pr, pr->u(r - 1), g, 0., pr->tsC, false, 0, s, pr->tsC * (F0 + r - 1)))) return rc;
             SP_CUDA(launch_convert(g, pr->u(r), pr->gc, pr->gt(pr->coarse_res), s));
         }
         for (int r = delta ? P - 1 : 0; r < P; ++r) {
