@@ -174,7 +174,13 @@ __global__ void __launch_bounds__(TY * TXP / 2, TY * TXP / 2 <= 256 ? 2 : 1)
 
     // thread -> cells (x0 + 2 px, x0 + 2 px + 1) of tile row `row`
     const int tid = threadIdx.x, px = tid % (TX / 2), row = tid / (TX / 2);
-    const bool leader = tid == 0;
+    // The thread that issues the copies.  With three pointwise slots (32 x 16 tiles;
+    // 64-column tiles have no room for a third) it sits in the last warp, which has no
+    // ring chunk and so reaches each plane's barrier early: 256^3 12.62 -> 12.56 ms per
+    // 40 steps, Parareal's fine sweep at 128^3 x 32 1 % faster; with two slots, whose
+    // next copy then waits behind that warp's own stencils, 256^3 was 1 % slower.
+    const bool leader = tid == (NP >= 3 ? S::NT - 32 : 0);
+    static_assert(NP < 3 || NH <= S::NT - 32, "the last warp has no ring chunk");
 
     pdl_trigger();  // the next kernel's CTAs may start as this grid's CTAs retire
     if (leader) {
@@ -575,7 +581,7 @@ template <int PAIR, int NW>
 cudaError_t set_pair_attrs() {
     cudaError_t e = set_pair_attr<PAIR, NW, 8, 7, 2, 64>();
     if (e == cudaSuccess) e = set_pair_attr<PAIR, NW, 16, 7, 2, 64>();
-    if (e == cudaSuccess) e = set_pair_attr<PAIR, NW, 16, 7, 2, 32>();
+    if (e == cudaSuccess) e = set_pair_attr<PAIR, NW, 16, 7, 3, 32>();
     return e;
 }
 
@@ -584,7 +590,7 @@ template <int PAIR, int NW>
 cudaError_t launch_pair_shape(const Geo& g4, const Geo& go, const PairLaunch& L, const Shape& sh, cudaStream_t s,
                               int* err) {
     add_launches(1);
-    if (sh.tx == 32 && sh.ty == 16) return launch_pair_T<PAIR, NW, 16, 7, 2, 32>(g4, go, L, sh, s, err);
+    if (sh.tx == 32 && sh.ty == 16) return launch_pair_T<PAIR, NW, 16, 7, 3, 32>(g4, go, L, sh, s, err);
     if (sh.tx == 64 && sh.ty == 8) return launch_pair_T<PAIR, NW, 8, 7, 2, 64>(g4, go, L, sh, s, err);
     if (sh.tx == 64 && sh.ty == 16) return launch_pair_T<PAIR, NW, 16, 7, 2, 64>(g4, go, L, sh, s, err);
     return cudaErrorInvalidValue;
