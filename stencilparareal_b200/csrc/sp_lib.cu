@@ -929,8 +929,10 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
     Tune best = h->tune(precision, batch);
     std::vector<int> zcs = {1, 2, 3, 4, 8, 16, 32, 64};
     zcs.push_back(g.nk);
-    float op_ms[kNumOps];
+    float op_ms[kNumOps], direct_ms[kNumOps];
+    Shape direct[kNumOps];  // the best direct shape of each stage
     for (auto& m : op_ms) m = 1e30f;
+    for (auto& m : direct_ms) m = 1e30f;
     for (int op : {OP_RK_S1, OP_RK_S2, OP_RK_S3, OP_RK_S4, OP_EULER}) {
         StageLaunch L;
         L.op = op;
@@ -964,9 +966,26 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
                         ms = std::min(ms, m);
                     }
                     if (ms < best_ms) { best_ms = ms; best.op[op] = sh; }
+                    if (kind == 0 && ms < direct_ms[op]) { direct_ms[op] = ms; direct[op] = sh; }
                 }
         op_ms[op] = best_ms;
     }
+    // RK4 steps whose four stages are all direct run as a chain without images, and
+    // overlap more than isolated timings show: they are taken unless those are more
+    // than 10 % worse than the best mixture's (128^3 FP64: chain 49 us per step, TMA 54),
+    // on the default's shape, measured in such chains, where that is direct (160^3
+    // FP32 50 us per step, with the isolated best of each stage 55-58)
+    float mixed = 0, chain = 0;
+    for (int op : {OP_RK_S1, OP_RK_S2, OP_RK_S3, OP_RK_S4}) {
+        mixed += op_ms[op];
+        chain += direct_ms[op];
+    }
+    const Shape dsh = default_stage_shape(g, batch);
+    if (wrap_supported(g) && chain < 1.1f * mixed)
+        for (int op : {OP_RK_S1, OP_RK_S2, OP_RK_S3, OP_RK_S4}) {
+            best.op[op] = dsh.tma ? direct[op] : dsh;
+            op_ms[op] = direct_ms[op];
+        }
     // fused stage pairs (FP64): best shape per pair, then fused or single-stage
     // steps by timing whole steps of both paths
     best.fused = best.cluster = 0;
@@ -1120,7 +1139,8 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
     }
     // small fields: the cluster-resident paths (z-slabs, (y,z) blocks) against
     // the best of the above, timed as they are used (a DoRK4 of a graph chunk of
-    // steps for one field; four batched steps for a batch)
+    // steps for one field; as many batched steps for a batch: a cluster launch loads
+    // and stores its fields once, which over four steps hid its advantage)
     if (precision == SP_F64 && (cluster_supported(g, 1) || cluster_supported(g, 2))) {
         int* err = h->err.as<int>();
         float path_ms[3] = {1e30f, 1e30f, 1e30f};
@@ -1138,10 +1158,10 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
                 if (c) {
                     ClusterLaunch L;
                     L.mode = c;
-                    L.in = p; L.out = p; L.items = batch; L.nsteps = 4; L.dt = dtt; L.nu = &nu; L.coef = h->coef;
+                    L.in = p; L.out = p; L.items = batch; L.nsteps = kChunk; L.dt = dtt; L.nu = &nu; L.coef = h->coef;
                     x = launch_rk4_cluster(g, L, s, err);
                 } else {
-                    for (int i = 0; i < 4 && x == cudaSuccess; ++i)
+                    for (int i = 0; i < kChunk && x == cudaSuccess; ++i)
                         x = enqueue_rk4_step(g, precision, h->coef, dtt, NuSrc{nu, nullptr}, p, p, p + fb, p + 2 * fb,
                                              p + 3 * fb, batch, nullptr, 0, tt, s, err);
                 }
