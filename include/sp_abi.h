@@ -313,7 +313,8 @@ int sp_store_violations(int* checked, long long* count);
  * Measurement support, no counterpart in the reference. */
 int sp_kernel_times(sp_convection* h, const double* field, double dt, int reps, int path, float* ms, int* count);
 /* Forces one launch shape for a precision and batch.  kind 0 or 1: every
- * single-stage kernel, ty in {4,8,16}, zchunk >= 1, RK4 steps unfused.  kind 2
+ * single-stage kernel, ty in {4,8,16} (kind 0: blocks of ty warps), zchunk >= 1, RK4
+ * steps unfused.  kind 2
  * (FP64): RK4 steps as fused pairs with ty in {8,16} and zchunk planes per CTA
  * (0 = automatic) on tiles of 64 columns; kind 4 the same on tiles of 32 x 16
  * cells (ty = 16; no wasted columns on grids such as 96^3).
