@@ -987,7 +987,8 @@ Shape default_stage_shape(const Geo& g, int items, bool adjoint) {
         sh.tma = 0;
         const bool wrap = wrap_supported(g);
         sh.ty = g.es == 8 && !wrap ? 8 : 4;
-        sh.zchunk = (int)std::min(wrap ? 2LL : 4LL, (threads + wave - 1) / wave);
+        // (no shorter than the launch grid's limit of 65535 chunks allows)
+        sh.zchunk = (int)std::max(std::min(wrap ? 2LL : 4LL, (threads + wave - 1) / wave), (g.nk + 65534) / 65535LL);
         return sh;
     }
     // TMA rings: 4-row tiles, z-chunks that give at least ~8 CTAs per SM

@@ -114,3 +114,26 @@ def test_adjoint_direct_equals_tma(sp, n):
         assert np.array_equal(got, want), tune
         assert np.allclose(gp, par, rtol=1e-9, atol=0), tune
         assert halo_ok(c, grad), tune
+
+
+@pytest.mark.parametrize("n,prec", [((4, 4, 140000), 0), ((8, 8, 150000), 1), ((2, 2, 70000), 0), ((3, 2, 300000), 0)])
+def test_default_path_on_long_grids(sp, n, prec):
+    """More planes than one launch has z-chunks of one or two planes (65535)."""
+    from stencilparareal_b200.adjoint import misfit_gradient
+    rng = np.random.default_rng(11)
+    q0 = rng.uniform(-1, 1, size=n[::-1])
+    c = sp.Convection(*n, 1.0, 0.02, 0.0, 0.3, -0.2, 0.25)
+    a, b = c.field(prec), c.field(prec)
+    got = []
+    for tune in (None, (4, 64, 1)):
+        if tune:
+            c.set_tune(prec, 1, *tune)
+        c.upload(a, q0)
+        c.DoRK4(a, b, 0.0, 1e-2, 2)
+        rk = c.download(b)
+        c.DoEuler(a, b, 0.0, 1e-2, 2)
+        got.append([rk, c.download(b)])
+        if prec == 0 and n[0] < 4:
+            got[-1].append(c.download(misfit_gradient(c, a, b, 0.0, 1e-2, 1)[1]))
+    for x, y in zip(*got):
+        assert np.array_equal(x, y)
