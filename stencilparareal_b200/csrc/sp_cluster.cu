@@ -799,6 +799,7 @@ cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_
     if ((L.mode == 2 ? !b2.cy : !nz) || L.nsteps < 1 || L.items < 1) return cudaErrorInvalidValue;
     if (!L.nutab && (L.nu_count < 1 || L.nu_count > kClusterNuSteps || (L.nu_count > 1 && L.nu_count < L.nsteps)))
         return cudaErrorInvalidValue;
+    if (!aligned16(L.in) || !aligned16(L.out)) return cudaErrorInvalidValue;
     ClusterArgs a{};
     a.in = static_cast<const double*>(L.in);
     a.out = static_cast<double*>(L.out);

@@ -661,6 +661,7 @@ Shape default_pair_shape(const Geo& g, int items) {
 cudaError_t launch_pair(const Geo& g4, const Geo& go, const PairLaunch& L, const Shape& sh, cudaStream_t s,
                         int* err) {
     if (!pair_supported(g4) || g4.halo != 4 || sh.zchunk < 0) return cudaErrorInvalidValue;
+    if (L.pair == 1 && !aligned16(L.out)) return cudaErrorInvalidValue;  // the others: as tensor maps
     if (!L.nu_items)
         return L.pair == 0 ? launch_pair_shape<0, 1>(g4, go, L, sh, s, err)
                            : launch_pair_shape<1, 1>(g4, go, L, sh, s, err);

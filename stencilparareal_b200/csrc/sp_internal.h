@@ -143,6 +143,10 @@ bool wrap_supported(const Geo& g);
 // kernel arguments, 104 bytes each: within 4 KB); larger batches take several.
 constexpr int kItemWeights = 32;
 
+// The stage, pair and cluster kernels access fields in 16-byte chunks: their launches
+// refuse a field that starts elsewhere.
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 // Launches one stage kernel; counts the launch.  err: device error word.
 cudaError_t launch_stage(const Geo& g, const StageLaunch& L, const Tune& t, cudaStream_t s, int* err);
 

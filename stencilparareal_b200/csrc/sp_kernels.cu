@@ -871,6 +871,9 @@ template <typename T, int OP, int NW>
 cudaError_t launch_op(const Geo& g, const StageLaunch& L, const Shape& t, cudaStream_t s, int* err) {
     if (L.wrap && (t.tma || !wrap_supported(g))) return cudaErrorInvalidValue;
     const KArgs<T> a = make_args<T>(g, L, t, err);
+    for (const void* p : {(const void*)a.yin, (const void*)a.yout, (const void*)a.aout, (const void*)a.pw0,
+                          (const void*)a.pw1, (const void*)a.pw2})
+        if (!aligned16(p)) return cudaErrorInvalidValue;
     if (!t.tma) return launch_direct_T<T, OP, NW>(g, L, a, t, s);
     switch (t.ty) {
         case 4: return launch_tma_T<T, OP, NW, 4, 5, 3>(g, L, a, t, s);

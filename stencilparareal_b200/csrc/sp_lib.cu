@@ -206,13 +206,15 @@ struct NuSrc {
     const double* items = nullptr;
 };
 
-// Whether a tune's RK4 (or Euler) steps run as a chain of wrapping direct kernels:
-// they read no periodic images and write none.
-bool wraps(const Geo& g, const Tune& t, bool rk) {
-    if (!wrap_supported(g)) return false;
+// Whether the stage kernels of a tune's RK4 (or Euler) steps are all direct ones.
+bool all_direct(const Tune& t, bool rk) {
     if (!rk) return !t.op[OP_EULER].tma;
     return !t.op[OP_RK_S1].tma && !t.op[OP_RK_S2].tma && !t.op[OP_RK_S3].tma && !t.op[OP_RK_S4].tma;
 }
+
+// Whether those steps run as a chain of wrapping direct kernels: they read no
+// periodic images and write none.
+bool wraps(const Geo& g, const Tune& t, bool rk) { return wrap_supported(g) && all_direct(t, rk); }
 
 bool wraps_adjoint(const Geo& g, const Tune& t) {
     return wrap_supported(g) && !t.op[OP_ADJ].tma && !t.op[OP_ADJ + 1].tma && !t.op[OP_ADJ + 2].tma &&
@@ -412,9 +414,24 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
     const Geo& g = h->g[prec];
     cudaStream_t s = h->stream();
     int* err = h->err.as<int>();
-    const Tune t = h->tune(prec, 1);
-    const bool const_nu = h->P.nufreq == 0.;
+    Tune t = h->tune(prec, 1);
+    // Fields that start off a 16-byte boundary, as a caller's view of a larger buffer may:
+    // the pairs read `in` cell by cell when they widen it, so without a tune they take
+    // it at every size; with a tune's direct shapes both fields are taken, by aligned
+    // copies.  The launches refuse the rest.
+    const bool tuned = h->tunes.count({prec, 1}) != 0;
+    if (!aligned16(in) && !tuned) t.no_small();
     const bool resident = rk && t.resident() && prec == 0 && cluster_supported(g, t.resident());
+    const bool pairs = !resident && rk && prec == 0 && t.pairs() && pair_supported(h->g4);
+    if (!(aligned16(in) && aligned16(out)) && tuned && !resident && !pairs && all_direct(t, rk)) {
+        if ((rc = h->ensure_scratch(prec, 2))) return rc;  // copies in fields 3 and 4 of the 2-item scratch
+        SP_CUDA(launch_periodicity(g, const_cast<void*>(in), 1, s));
+        SP_CUDA(cudaMemcpyAsync(h->sbuf(prec, 3, 1), in, g.total * g.es, cudaMemcpyDeviceToDevice, s));
+        if ((rc = do_prop(h, prec, rk, h->sbuf(prec, 3, 1), h->sbuf(prec, 4, 1), tStart, dt, n))) return rc;
+        SP_CUDA(cudaMemcpyAsync(out, h->sbuf(prec, 4, 1), g.total * g.es, cudaMemcpyDeviceToDevice, s));
+        return SP_OK;
+    }
+    const bool const_nu = h->P.nufreq == 0.;
     // Periodicity on the input, in place, as before the reference's first stencil
     // (the cluster-resident path writes the images of its input itself).
     if (!resident) SP_CUDA(launch_periodicity(g, const_cast<void*>(in), 1, s));
@@ -438,7 +455,7 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
                 nus[k] = computenu(h->P.nu0, h->P.nufreq, i + k == 0 ? tStart : tStart + (i + k) * dt);
             SP_CUDA(launch_rk4_cluster(g, L, s, err));
         }
-    } else if (rk && t.pairs() && prec == 0 && pair_supported(h->g4)) {
+    } else if (pairs) {
         // fused stage pairs: widen the input once, alternate the step-start
         // field between wbuf(0) and wbuf(1), write the last step to `out`
         if ((rc = h->ensure_wide(1))) return rc;
@@ -503,7 +520,7 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
             SP_CUDA(cudaMemcpyAsync(out, src, g.total * g.es, cudaMemcpyDeviceToDevice, s));
         }
     }
-    if (!resident && !(rk && prec == 0 && t.pairs() && pair_supported(h->g4)) && wraps(g, t, rk))
+    if (!resident && !pairs && wraps(g, t, rk))
         SP_CUDA(launch_periodicity(g, out, 1, s));  // the wrapping kernels wrote no images
     return SP_OK;
 }
