@@ -298,8 +298,8 @@ int sp_autotune(sp_convection* h, int precision, int batch);
 int sp_selftest_wait_timeout(sp_convection* h, double limit_ms);
 /* Store-bounds checking, the stand-in for a memory sanitizer: in the library
  * built with -DSP_BOUNDS_CHECK=1 (libstencilparareal_checked.so) every global
- * store of the stencil-producing kernels (stage, fused-pair and widening
- * kernels) is tested against its output allocation and skipped, not made, when
+ * store of the stencil-producing kernels (stage, fused-pair, widening and
+ * cluster-resident kernels) is tested against its output allocation and skipped, not made, when
  * it falls outside.  *checked = 1 in that build, 0 otherwise; *count = such
  * stores on the current device since the previous call (then reset), after
  * waiting for the device.  No counterpart in the reference. */

@@ -771,6 +771,14 @@ cudaError_t prepare_cluster_kernels() {
 
 }  // namespace
 
+unsigned long long take_store_violations_cluster() {
+    unsigned int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_store_violations, sizeof v) != cudaSuccess) return 0;
+    const unsigned int zero = 0;
+    cudaMemcpyToSymbol(g_store_violations, &zero, sizeof zero);
+    return v;
+}
+
 bool cluster_supported(const Geo& g, int mode) {
     return mode == 2 ? blocks_2d(g, 1).cy != 0 : cluster_nz(g) != 0;
 }

@@ -792,7 +792,8 @@ extern "C" int sp_store_violations(int* checked, long long* count) {
     *checked = 0;
 #endif
     SP_CUDA(cudaDeviceSynchronize());
-    *count = (long long)(take_store_violations_stages() + take_store_violations_pairs());
+    *count = (long long)(take_store_violations_stages() + take_store_violations_pairs() +
+                         take_store_violations_cluster());
     return SP_OK;
 }
 

@@ -106,3 +106,45 @@ def test_release_build_reports_unchecked(sp):
     chk, cnt = C.c_int(-1), C.c_longlong(-1)
     assert sp._lib.lib().sp_store_violations(C.byref(chk), C.byref(cnt)) == sp._lib.SP_OK
     assert chk.value == 0 and cnt.value == 0
+
+
+CLUSTER_SCRIPT = r"""
+import ctypes as C, json, sys
+sys.path.insert(0, {root!r}); sys.path.insert(0, {tests!r})
+import stencilparareal_b200 as sp
+from ics import gaussian_noise
+L = sp._lib
+for n, kinds in (((16, 16, 8), (3, 5)), ((24, 20, 12), (3, 5)), ((30, 30, 9), (3, 5)), ((16, 13, 16), (3,)),
+                 ((24, 24, 24), (None,))):
+    q0 = gaussian_noise(*n, seed=1)
+    for nufreq in (0.0, 30.0):
+        for kind in kinds:
+            c = sp.Convection(*n, 1.0 / n[0], 0.02, nufreq, 1.0, -0.5, 0.25)
+            if kind:
+                c.set_tune(sp.SP_F64, 1, 0, 0, kind)
+            fi, fo = c.field(), c.field()
+            c.upload(fi, q0)
+            before = sp.launch_count()
+            c.DoRK4(fi, fo, 0.0, 1e-4, 3)
+            c.DoRK4(fo, fo, 0.0, 1e-4, 3)
+            c.synchronize()
+            assert sp.launch_count() - before == 2  # cluster-resident
+chk, cnt = C.c_int(), C.c_longlong()
+L.check(L.lib().sp_store_violations(C.byref(chk), C.byref(cnt)))
+print(json.dumps({{"checked": chk.value, "count": cnt.value}}))
+"""
+
+
+@pytest.mark.parametrize("shrink", [0, 1])
+def test_cluster_stores_are_checked(checked_lib, shrink):
+    """The cluster kernels' results and periodic images (both fields), constant and
+    varying diffusivity: inside their allocations, and counted when the bounds are
+    narrowed by one plane."""
+    env = dict(os.environ, STENCILPARAREAL_LIB=checked_lib)
+    if shrink:
+        env["SP_BOUNDS_SHRINK_PLANES"] = str(shrink)
+    script = CLUSTER_SCRIPT.format(root=ROOT, tests=os.path.join(ROOT, "tests"))
+    r = subprocess.run([sys.executable, "-c", script], env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    out = json.loads(r.stdout.strip().splitlines()[-1])
+    assert out["checked"] == 1 and (out["count"] > 0) == bool(shrink)
