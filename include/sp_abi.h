@@ -307,8 +307,9 @@ int sp_store_violations(int* checked, long long* count);
 /* Median duration in ms of each kernel of an FP64 RK4 step, timed with CUDA
  * events around every launch on the handle's stream over `reps` steps (after
  * one untimed step; all steps enqueued before one synchronisation) run on a
- * copy of `field` (which is left unchanged).  path 0: the kernels the handle's
- * tune runs, 1: the four stage kernels (tuned shapes), 2: the fused pairs.
+ * copy of `field` (which is left unchanged).  path 0: the kernels sp_do_rk4 runs
+ * (where it runs cluster-resident, one kernel for all steps: those its steps would
+ * run on otherwise), 1: the four stage kernels (shapes in use), 2: the fused pairs.
  * *count = 2 (ms[0..1]: pairs 1+2, 3+4) or 4 (ms[0..3]: stages S1..S4).
  * Measurement support, no counterpart in the reference. */
 int sp_kernel_times(sp_convection* h, const double* field, double dt, int reps, int path, float* ms, int* count);

@@ -206,7 +206,8 @@ class Convection:
         """Average ms of each kernel of an FP64 RK4 step (CUDA events on the
         library's stream), run on a copy of `field`: {"P12", "P34"} for the fused
         pairs, {"S1".."S4"} for the stage kernels.  path: "tuned" (what DoRK4
-        runs), "stages" or "pairs"."""
+        runs; where that is the cluster-resident kernel, the kernels its steps
+        would run on otherwise), "stages" or "pairs"."""
         ms = (C.c_float * 4)()
         cnt = C.c_int()
         code = {"tuned": 0, "stages": 1, "pairs": 2}[path]

@@ -821,7 +821,9 @@ extern "C" int sp_kernel_times(sp_convection* h, const double* field, double dt,
     int* err = h->err.as<int>();
     std::vector<float> times[4];  // per kernel, one duration per timed rep
     if (path == 2 && !pair_supported(h->g4)) return fail(SP_ERR_INVALID, "fused pairs need >= 4 cells per axis");
-    const bool fused = path == 2 || (path == 0 && t.fused && pair_supported(h->g4));
+    // path 0: what sp_do_rk4 launches; a cluster-resident tune, whose steps are one
+    // kernel, gets the kernels its steps would run on otherwise
+    const bool fused = path == 2 || (path == 0 && (t.resident() ? t.fused : t.pairs()) && pair_supported(h->g4));
     if (fused) {
         if ((rc = h->ensure_wide(1))) return rc;
     } else if ((rc = h->ensure_scratch(0, 2))) {  // fields 0, 3, 4, 5 of the 2-item scratch
@@ -860,6 +862,7 @@ extern "C" int sp_kernel_times(sp_convection* h, const double* field, double dt,
         if (e == cudaSuccess) e = cudaMemcpyAsync(q, field, g.total * g.es, cudaMemcpyDeviceToDevice, s);
         StageLaunch L;
         L.prec = 0; L.items = 1; L.nu = nu; L.coef = h->coef;
+        L.wrap = wraps(g, t, true);
         const double dthalf = dt * .5;
         const int op[4] = {OP_RK_S1, OP_RK_S2, OP_RK_S3, OP_RK_S4};
         const void* yin[4] = {q, ya, yb, ya};

@@ -137,3 +137,22 @@ def test_default_path_on_long_grids(sp, n, prec):
             got[-1].append(c.download(misfit_gradient(c, a, b, 0.0, 1e-2, 1)[1]))
     for x, y in zip(*got):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n,tune", [((64, 64, 64), None), ((47, 40, 36), None), ((160, 144, 140), None),
+                                    ((160, 160, 160), None), ((48, 40, 36), (8, 2, 0)), ((48, 40, 36), (16, 0, 4))])
+def test_kernel_times_names_the_kernels_that_run(sp, n, tune):
+    """As many kernels as DoRK4 launches per step: two pairs or four stages."""
+    c = conv_of(sp, n)
+    if tune:
+        c.set_tune(sp.SP_F64, 1, *tune)
+    a, b = c.field(), c.field()
+    c.upload(a, gaussian_noise(*n, seed=3))
+    counts = []
+    for k in (3, 4):
+        before = sp.launch_count()
+        c.DoRK4(a, b, 0.0, 1e-5, k)
+        counts.append(sp.launch_count() - before)
+    before = b.data.clone()
+    assert len(c.kernel_times(a, 1e-5, reps=2)) == counts[1] - counts[0]
+    assert bool((b.data == before).all())
