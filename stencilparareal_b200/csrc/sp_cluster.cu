@@ -816,7 +816,6 @@ cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_
     a.px = g.px;
     a.plane = g.plane;
     a.ni = g.ni; a.nj = g.nj; a.nk = g.nk;
-    a.nsteps = L.nsteps;
     a.items = L.items;
     const bool vary = L.nutab || L.nu_count > 1;
     if (!vary) fill_w13(a.w, L.coef, L.nu[0]);
@@ -836,7 +835,6 @@ cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_
     a.sb = out_bounds(L.out, g, L.items);
     a.cy = b2.cy;
     a.cz = b2.cz;
-    add_launches(1);
     const int upt = (long long)(g.ni / 2) * g.nj > kClusterThreads ? 2 : 1;
     auto launch = [&](auto k) {
         return L.mode == 2 ? launch_clusters(k, b2.cy * b2.cz, b2.nt,
@@ -844,10 +842,22 @@ cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_
                            : launch_clusters(k, g.nk / nz, kClusterThreads,
                                              16 + (size_t)2 * (nz + 4) * g.ni * g.nj * 8, a, s);
     };
-    if (L.mode == 2)
-        return vary ? with_block_kernel<true>(b2.zt, b2.upt, b2.nt, launch)
-                    : with_block_kernel<false>(b2.zt, b2.upt, b2.nt, launch);
-    return vary ? with_slab_kernel<true>(nz, upt, launch) : with_slab_kernel<false>(nz, upt, launch);
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < L.nsteps && e == cudaSuccess; i += a.nsteps) {
+        a.nsteps = std::min(L.nsteps - i, kClusterMaxSteps);
+        if (i) {
+            a.in = a.out;
+            a.in_images = nullptr;
+            if (a.nutab) a.nutab += (long long)kClusterMaxSteps * a.items;
+        }
+        add_launches(1);
+        if (L.mode == 2)
+            e = vary ? with_block_kernel<true>(b2.zt, b2.upt, b2.nt, launch)
+                     : with_block_kernel<false>(b2.zt, b2.upt, b2.nt, launch);
+        else
+            e = vary ? with_slab_kernel<true>(nz, upt, launch) : with_slab_kernel<false>(nz, upt, launch);
+    }
+    return e;
 }
 
 }  // namespace sp

@@ -107,7 +107,10 @@ struct StageLaunch {
 // the interiors of `items` fields at `in`, writes the results with their periodic
 // images at `out` (in == out allowed).  Step i uses the diffusivity nu[i] (nu[0] in
 // every step if nu_count is 1), or nutab[i * items + b] for item b.
+// One launch takes at most kClusterMaxSteps steps (a second at the largest sizes, and the
+// kernels count stages in an int); longer runs take several.
 constexpr int kClusterNuSteps = 256;
+constexpr int kClusterMaxSteps = 1 << 16;
 struct ClusterLaunch {
     const void* in = nullptr;
     void* out = nullptr;

@@ -167,3 +167,36 @@ def test_default_small_path_equals_stage_kernels(sp, n, P, nufreq):
     assert np.array_equal(got[0][0], got[1][0])
     if P == 1:  # the input's halo was refreshed in place
         assert torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("kind", [None, 3, 5])
+def test_long_runs_take_several_launches(sp, kind):
+    """More steps than one launch takes (65536): the same field as in two calls."""
+    n, steps, cut = (8, 12, 8), 65536 + 70, 300
+    c = _conv(sp, n)
+    if kind:
+        c.set_tune(sp.SP_F64, 1, 0, 0, kind)
+    a, b, d = c.field(), c.field(), c.field()
+    c.upload(a, fourier_modes(*n, seed=6))
+    before = sp.launch_count()
+    c.DoRK4(a, b, 0.0, 1e-6, steps)
+    assert sp.launch_count() - before == 2
+    c.DoRK4(a, d, 0.0, 1e-6, cut)
+    c.DoRK4(d, d, 0.0, 1e-6, steps - cut)
+    assert np.isfinite(c.download(b)).all() and torch.equal(b.data, d.data)
+
+
+def test_long_fine_sweep_with_one_diffusivity_per_step(sp):
+    """A fine sweep of more steps per slice than one launch takes reads its table of
+    diffusivities on from where the launch before ended.  After as many iterations as
+    slices the result is the serial run's (to rounding; nu is 7 % off in the last 30
+    steps of a slice, 1e-6 in the field, if the table is read from its start again)."""
+    n, P, steps = (8, 6, 8), 2, 65536 + 30
+    c = _conv(sp, n, nufreq=50.0)
+    conf = sp.RuntimeConfiguration(timeSlices=P, nu0=0.02, nufreq=50.0, cy=-0.5, cz=0.25, gridSize=8,
+                                   endTime=1e-6 * P * steps, timeStepsFine=P * steps, timeStepsCoarse=P, kmax=P)
+    a, b, d = c.field(), c.field(), c.field()
+    c.upload(a, fourier_modes(*n, seed=7))
+    sp.Parareal(c, a, b, 0.0, conf, coarse="rk4", coarse_precision="f64").DoParallel()
+    c.DoRK4(a, d, 0.0, 1e-6, P * steps)
+    assert rel_l2(c.download(b), c.download(d)) < 1e-9
