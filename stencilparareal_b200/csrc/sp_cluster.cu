@@ -58,10 +58,11 @@ struct ClusterArgs {
     int ni, nj, nk;
     int nsteps;
     W13<double> w;            // weights of every step (one diffusivity)
-    const double* nutab;      // VARY: step i of item b takes nutab[i * items + b] ...
+    int vary;                 // 1: one diffusivity per step instead:
+    const double* nutab;      // step i of item b takes nutab[i * items + b] ...
     double nu[kClusterNuSteps];  // ... or (nutab null) nu[i]
     int items;
-    double ca[3], s4;         // VARY: coefficients of R (Coef)
+    double ca[3], s4;         // vary: coefficients of R (Coef)
     double dthalf, dt, dt3, dt6;
     const int* item_lo;
     int item_base;
@@ -88,6 +89,14 @@ __device__ __forceinline__ void step_weights(W13<double>& w, const ClusterArgs& 
     w.c = __dmul_rn(-90., nl);
 }
 
+// Where a kernel has its weights: in the constant bank (one diffusivity), worked out
+// each step (one per step), or in registers, replaced each step if they vary.  The
+// bank is the fastest where little spills (32 x 32 x 48 on slabs 6.39 against 6.55 ms
+// per 1000 steps in registers, 30^3 on blocks 4.89 / 4.97).  The forms at their register cap need more registers
+// with it, for fetching each weight again beside the operands: 32^3 4.55 / 4.36, 36^3
+// 14.1 / 12.5 and 40^3 14.8 / 12.0 on blocks, 20 x 20 x 40 4.64 / 4.33 on slabs of four planes.
+enum Source { BANK, STEP, EITHER };
+
 // Periodic images of the cell pair (x, y, z) within two cells of a face -- on faces,
 // edges and corners, as Periodicity leaves them (p: the pair's address in its field).
 __device__ __forceinline__ void pair_images(const StoreBounds& b, double* p, const ClusterArgs& a, int x, int y, int z,
@@ -107,9 +116,40 @@ __device__ __forceinline__ void pair_images(const StoreBounds& b, double* p, con
     }
 }
 
+// Refreshes the images of the input from this CTA's cells: `rows` rows from y0 on of
+// `planes` planes from z0 on, U pairs at a time (their loads overlap; one at a time a
+// call of one step on 32^3 took 17.6 us, four 16.6).  Ahead of the run, for the kernels
+// that hold their weights in registers: done with the loads of the run's fields,
+// which then loads nothing twice, it cost them 2 % for the whole run (40^3 on blocks 12.35 /
+// 12.02 ms per 1000 steps).
+template <int NT, int U>
+__device__ __forceinline__ void input_images(const ClusterArgs& a, int item, int y0, int rows, int z0, int planes) {
+    const long long base = (long long)item * a.item_stride + a.origin;
+    const unsigned half = (unsigned)a.ni / 2u, per = half * (unsigned)rows, n = per * (unsigned)planes;
+#pragma unroll 1
+    for (unsigned c0 = threadIdx.x; c0 < n; c0 += U * NT) {
+        V2 v[U];
+        int x[U], y[U], z[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const unsigned c = c0 + k * NT, o = c / per, u = c - o * per, r = u / half;
+            x[k] = 2 * (int)(u - r * half);
+            y[k] = y0 + (int)r;
+            z[k] = z0 + (int)o;
+            const bool edge = x[k] < 2 || x[k] >= a.ni - 2 || y[k] < 2 || y[k] >= a.nj - 2 || z[k] < 2 || z[k] >= a.nk - 2;
+            if (c >= n || !edge) z[k] = -1;  // no image
+            else v[k] = ld16<double>(a.in + base + z[k] * a.plane + y[k] * a.px + x[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+            if (z[k] >= 0)
+                pair_images(a.sb_in, a.in_images + base + z[k] * a.plane + y[k] * a.px + x[k], a, x[k], y[k], z[k], v[k]);
+    }
+}
+
 // Cluster of C = nk / NZ CTAs per field (NZ >= 2, C >= 2); UPT units of two
 // x-adjacent cells of one row per thread, every own plane of each unit.
-template <int NZ, int UPT, bool VARY>
+template <int NZ, int UPT, Source SRC>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid_constant__ ClusterArgs a) {
     constexpr int NPL = NZ + 4;  // planes per buffer: 2 halo, NZ own, 2 halo
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -131,6 +171,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
     const uint32_t lower = (rank + C - 1) % C, upper = (rank + 1) % C;
     const int z0 = (int)rank * NZ;
     const double* fin = a.in + (long long)item * a.item_stride + a.origin;
+
+    constexpr bool kImagesFirst = SRC == EITHER;
+    if (kImagesFirst && a.in_images) input_images<kClusterThreads, 2>(a, item, 0, nj, z0, NZ);
 
     const int tid = threadIdx.x;
     if (tid == 0) {
@@ -191,7 +234,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
             sts2(base0 + (uint32_t)((p * plane_cells + uy[j] * ni + ux[j]) * 8), v);
             if (p >= 2 && p < NZ + 2) {
                 q[j][p - 2] = v;
-                if (a.in_images)
+                if (!kImagesFirst && a.in_images)
                     pair_images(a.sb_in, a.in_images + (long long)item * a.item_stride + a.origin +
                                              (long long)z * a.plane + (long long)uy[j] * a.px + ux[j],
                                 a, ux[j], uy[j], z, v);
@@ -206,10 +249,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
 
     bool bad = false;
     const int nstage = 4 * a.nsteps;
-    [[maybe_unused]] W13<double> wv;  // VARY: this step's weights; else they stay in the constant bank
+    [[maybe_unused]] W13<double> wv;  // this step's weights (unless they stay in the constant bank)
+    if constexpr (SRC == EITHER) wv = a.w;
     const W13<double>& w = [&]() -> const W13<double>& {
-        if constexpr (VARY) return wv;
-        else return a.w;
+        if constexpr (SRC == BANK) return a.w;
+        else return wv;
     }();
     // halo bytes per stage: two planes from each z-neighbour
     const uint32_t halo_bytes = 4u * (uint32_t)plane_cells * 8u;
@@ -323,7 +367,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
         __syncthreads();
     };
     for (int i = 0; i < a.nsteps; ++i) {
-        if constexpr (VARY) step_weights(wv, a, i, item);
+        if constexpr (SRC != BANK)
+            if (SRC == STEP || a.vary) step_weights(wv, a, i, item);
         stage(std::integral_constant<int, 0>{}, 4 * i);
         stage(std::integral_constant<int, 1>{}, 4 * i + 1);
         stage(std::integral_constant<int, 2>{}, 4 * i + 2);
@@ -364,7 +409,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_rk4_cluster(const __grid
 // NT threads per CTA: 256 (up to 255 registers, one unit per thread) where the
 // block's units fit, else 512 (128 registers, up to two units per thread); at
 // 32^3 and 24^3 the 256-thread form is ~14 % faster, at 40^3 it would spill.
-template <int ZT, int UPT, int NT, bool VARY>
+template <int ZT, int UPT, int NT, Source SRC>
 __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__ ClusterArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);  // 2 mbarriers (stage parity)
@@ -391,6 +436,9 @@ __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__
     const int ry = (int)rank % cy, rz = (int)rank / cy;
     const int y0 = ry * BY, z0 = rz * BZ;
     const double* fin = a.in + (long long)item * a.item_stride + a.origin;
+
+    constexpr bool kImagesFirst = SRC == EITHER;
+    if (kImagesFirst && a.in_images) input_images<NT, 4>(a, item, y0, BY, z0, BZ);
 
     const int tid = threadIdx.x;
     if (tid == 0) {
@@ -454,7 +502,7 @@ __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__
             const int y = y0 + uy[j], z = z0 + uz[j] + o;
             const long long at = (long long)z * a.plane + (long long)y * a.px + ux[j];
             q[j][o] = ld16<double>(fin + at);
-            if (a.in_images)
+            if (!kImagesFirst && a.in_images)
                 pair_images(a.sb_in, a.in_images + (long long)item * a.item_stride + a.origin + at, a, ux[j], y, z,
                             q[j][o]);
         }
@@ -463,10 +511,11 @@ __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__
 
     bool bad = false;
     const int nstage = 4 * a.nsteps;
-    [[maybe_unused]] W13<double> wv;  // VARY: this step's weights; else they stay in the constant bank
+    [[maybe_unused]] W13<double> wv;  // this step's weights (unless they stay in the constant bank)
+    if constexpr (SRC == EITHER) wv = a.w;
     const W13<double>& w = [&]() -> const W13<double>& {
-        if constexpr (VARY) return wv;
-        else return a.w;
+        if constexpr (SRC == BANK) return a.w;
+        else return wv;
     }();
     const uint32_t halo_bytes = (uint32_t)(4 * BY + 4 * BZ) * row_bytes;
     const uint32_t yshift = (uint32_t)BY * row_bytes, zshift = (uint32_t)BZ * plane_bytes;
@@ -554,7 +603,8 @@ __global__ void __launch_bounds__(NT, 1) k_rk4_cluster2d(const __grid_constant__
         __syncthreads();
     };
     for (int i = 0; i < a.nsteps; ++i) {
-        if constexpr (VARY) step_weights(wv, a, i, item);
+        if constexpr (SRC != BANK)
+            if (SRC == STEP || a.vary) step_weights(wv, a, i, item);
         stage(std::integral_constant<int, 0>{}, 4 * i);
         stage(std::integral_constant<int, 1>{}, 4 * i + 1);
         stage(std::integral_constant<int, 2>{}, 4 * i + 2);
@@ -625,7 +675,7 @@ int resident_clusters(int C) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_rk4_cluster<2, 1, false>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, k_rk4_cluster<2, 1, BANK>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;  // asked again next time
     }
@@ -668,15 +718,20 @@ int cluster_nz(const Geo& g, int items = 1, double* us = nullptr) {
 }
 
 // f(<kernel>) for the slab kernel of NZ planes per CTA and UPT units per thread.
-template <bool VARY, typename F>
-cudaError_t with_slab_kernel(int nz, int upt, F&& f) {
+template <int NZ, int UPT, typename F>
+cudaError_t with_slab_form(bool vary, F&& f) {
+    if constexpr (NZ == 4) return f(k_rk4_cluster<NZ, UPT, EITHER>);
+    else return vary ? f(k_rk4_cluster<NZ, UPT, STEP>) : f(k_rk4_cluster<NZ, UPT, BANK>);
+}
+template <typename F>
+cudaError_t with_slab_kernel(bool vary, int nz, int upt, F&& f) {
     switch (nz * 2 + upt - 1) {
-        case 4: return f(k_rk4_cluster<2, 1, VARY>);
-        case 5: return f(k_rk4_cluster<2, 2, VARY>);
-        case 6: return f(k_rk4_cluster<3, 1, VARY>);
-        case 7: return f(k_rk4_cluster<3, 2, VARY>);
-        case 8: return f(k_rk4_cluster<4, 1, VARY>);
-        case 9: return f(k_rk4_cluster<4, 2, VARY>);
+        case 4: return with_slab_form<2, 1>(vary, f);
+        case 5: return with_slab_form<2, 2>(vary, f);
+        case 6: return with_slab_form<3, 1>(vary, f);
+        case 7: return with_slab_form<3, 2>(vary, f);
+        case 8: return with_slab_form<4, 1>(vary, f);
+        case 9: return with_slab_form<4, 2>(vary, f);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -735,37 +790,42 @@ Blocks2d blocks_2d(const Geo& g, int items) {
 }
 
 // f(<kernel>) for the thread form of a block shape.
-template <bool VARY, typename F>
-cudaError_t with_block_kernel(int zt, int upt, int nt, F&& f) {
+template <int ZT, int UPT, int NT, typename F>
+cudaError_t with_block_form(bool vary, F&& f) {
+    if constexpr (UPT == 2) return f(k_rk4_cluster2d<ZT, UPT, NT, EITHER>);
+    else if (vary) return f(k_rk4_cluster2d<ZT, UPT, NT, STEP>);  // (32^3 with nu(t) 4.36 ms, 4.45 on EITHER)
+    else return f(k_rk4_cluster2d<ZT, UPT, NT, ZT == 4 ? EITHER : BANK>);
+}
+template <typename F>
+cudaError_t with_block_kernel(bool vary, int zt, int upt, int nt, F&& f) {
     if (nt == 256) {
         switch (zt) {
-            case 1: return f(k_rk4_cluster2d<1, 1, 256, VARY>);
-            case 2: return f(k_rk4_cluster2d<2, 1, 256, VARY>);
-            case 4: return f(k_rk4_cluster2d<4, 1, 256, VARY>);
+            case 1: return with_block_form<1, 1, 256>(vary, f);
+            case 2: return with_block_form<2, 1, 256>(vary, f);
+            case 4: return with_block_form<4, 1, 256>(vary, f);
             default: return cudaErrorInvalidValue;
         }
     }
     switch (zt * 2 + upt - 1) {
-        case 2: return f(k_rk4_cluster2d<1, 1, 512, VARY>);
-        case 3: return f(k_rk4_cluster2d<1, 2, 512, VARY>);
-        case 4: return f(k_rk4_cluster2d<2, 1, 512, VARY>);
-        case 5: return f(k_rk4_cluster2d<2, 2, 512, VARY>);
+        case 2: return with_block_form<1, 1, 512>(vary, f);
+        case 3: return with_block_form<1, 2, 512>(vary, f);
+        case 4: return with_block_form<2, 1, 512>(vary, f);
+        case 5: return with_block_form<2, 2, 512>(vary, f);
         default: return cudaErrorInvalidValue;
     }
 }
 
-template <bool VARY>
-cudaError_t prepare_cluster_kernels() {
+cudaError_t prepare_cluster_kernels(bool vary) {
     auto set = [](auto k) { return set_attr_cluster(k); };
     cudaError_t e = cudaSuccess;
     for (int nz = 2; nz <= 4; ++nz)
         for (int upt = 1; upt <= 2; ++upt)
-            if (e == cudaSuccess) e = with_slab_kernel<VARY>(nz, upt, set);
+            if (e == cudaSuccess) e = with_slab_kernel(vary, nz, upt, set);
     for (int zt : {1, 2, 4})
-        if (e == cudaSuccess) e = with_block_kernel<VARY>(zt, 1, 256, set);
+        if (e == cudaSuccess) e = with_block_kernel(vary, zt, 1, 256, set);
     for (int zt = 1; zt <= 2; ++zt)
         for (int upt = 1; upt <= 2; ++upt)
-            if (e == cudaSuccess) e = with_block_kernel<VARY>(zt, upt, 512, set);
+            if (e == cudaSuccess) e = with_block_kernel(vary, zt, upt, 512, set);
     return e;
 }
 
@@ -797,8 +857,8 @@ int default_cluster_mode(const Geo& g, int items) {
 }
 
 cudaError_t prepare_cluster() {
-    const cudaError_t e = prepare_cluster_kernels<false>();
-    return e != cudaSuccess ? e : prepare_cluster_kernels<true>();
+    const cudaError_t e = prepare_cluster_kernels(false);
+    return e != cudaSuccess ? e : prepare_cluster_kernels(true);
 }
 
 cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_t s, int* err) {
@@ -818,6 +878,7 @@ cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_
     a.ni = g.ni; a.nj = g.nj; a.nk = g.nk;
     a.items = L.items;
     const bool vary = L.nutab || L.nu_count > 1;
+    a.vary = vary;
     if (!vary) fill_w13(a.w, L.coef, L.nu[0]);
     a.nutab = L.nutab;
     if (!L.nutab) std::copy(L.nu, L.nu + L.nu_count, a.nu);
@@ -852,10 +913,9 @@ cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_
         }
         add_launches(1);
         if (L.mode == 2)
-            e = vary ? with_block_kernel<true>(b2.zt, b2.upt, b2.nt, launch)
-                     : with_block_kernel<false>(b2.zt, b2.upt, b2.nt, launch);
+            e = with_block_kernel(vary, b2.zt, b2.upt, b2.nt, launch);
         else
-            e = vary ? with_slab_kernel<true>(nz, upt, launch) : with_slab_kernel<false>(nz, upt, launch);
+            e = with_slab_kernel(vary, nz, upt, launch);
     }
     return e;
 }

@@ -200,3 +200,26 @@ def test_long_fine_sweep_with_one_diffusivity_per_step(sp):
     sp.Parareal(c, a, b, 0.0, conf, coarse="rk4", coarse_precision="f64").DoParallel()
     c.DoRK4(a, d, 0.0, 1e-6, P * steps)
     assert rel_l2(c.download(b), c.download(d)) < 1e-9
+
+
+@pytest.mark.parametrize("nufreq", [0.0, 30.0])
+@pytest.mark.parametrize("n,kind", [((32, 32, 32), 5), ((24, 24, 24), 5), ((16, 16, 16), 5), ((30, 30, 30), 5),
+                                    ((36, 36, 36), 5), ((40, 40, 40), 5), ((24, 32, 48), 5), ((4, 4, 4), 5),
+                                    ((16, 16, 44), 3), ((40, 40, 40), 3), ((36, 36, 36), 3), ((32, 16, 48), 3),
+                                    ((24, 24, 24), None)])
+def test_every_form_leaves_both_halos_as_periodicity_does(sp, n, kind, nufreq):
+    """Every source of the weights, and both ways of refreshing the input's images: the
+    whole buffers, halos included, of a run on the stage kernels and of Periodicity."""
+    got = []
+    for k in (kind, 1):
+        c = _conv(sp, n, nufreq=nufreq)
+        if k:
+            c.set_tune(sp.SP_F64, 1, *((0, 0, k) if k != 1 else (4, 8, 1)))
+        a, b = c.field(), c.field()
+        c.upload(a, gaussian_noise(*n, seed=8))
+        c.DoRK4(a, b, 0.1, 1e-5, 5)
+        if k == 1:
+            c.Periodicity(b)
+        got.append((a.data.clone(), b.data.clone()))
+    assert torch.equal(got[0][0], got[1][0])
+    assert torch.equal(got[0][1], got[1][1])
