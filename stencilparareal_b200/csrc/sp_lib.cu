@@ -78,7 +78,11 @@ struct DevBuf {
         if (n <= bytes && p) return cudaSuccess;
         release();
         cudaError_t e = cudaMalloc(&p, n);
-        if (e != cudaSuccess) { p = nullptr; return e; }
+        if (e != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();  // reported here, not by a later launch
+            return e;
+        }
         bytes = n;
         e = cudaMemset(p, 0, n);
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -164,10 +168,19 @@ struct sp_convection {
             if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
         graphs.clear();
     }
+    // Stage-kernel runs with graph chunks of fields up to 128 MB keep the state between
+    // steps in a work field of the handle (the last one of its scratch), so that the
+    // graph holds no caller's address: captured and instantiated again for every new
+    // output (200 nodes), 60 steps of 64^3 took 1.55 ms on a new field and 0.80 on one that
+    // was seen.  Larger fields take longer than that over one step, and the work field
+    // would be felt.
+    bool keeps_state(int prec) const { return (size_t)g[prec].total * g[prec].es <= (size_t)128 << 20; }
+    void* state(int prec) const { return sbuf(prec, 3 * scratch_items[prec], 1); }
     int ensure_scratch(int prec, int items) {
         if (scratch_items[prec] >= items) return SP_OK;
         drop_graphs();  // captured graphs hold the old scratch addresses
-        const size_t n = (size_t)3 * items * g[prec].total * g[prec].es;
+        const size_t n = ((size_t)3 * items + (keeps_state(prec) ? 1 : 0)) * g[prec].total * g[prec].es;
+        scratch_items[prec] = 0;  // a failing allocation leaves none
         cudaError_t e = scratch[prec].alloc(n);
         if (e != cudaSuccess) return fail(SP_ERR_NOMEM, "scratch allocation of %zu bytes: %s", n, cudaGetErrorString(e));
         scratch_items[prec] = items;
@@ -177,6 +190,7 @@ struct sp_convection {
         if (wide_items >= items) return SP_OK;
         drop_graphs();
         const size_t n = (size_t)3 * items * g4.total * g4.es;
+        wide_items = 0;
         cudaError_t e = wide.alloc(n);
         if (e != cudaSuccess) return fail(SP_ERR_NOMEM, "fused-pair fields of %zu bytes: %s", n, cudaGetErrorString(e));
         wide_items = items;
@@ -410,7 +424,6 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
     if (!in || !out) return fail(SP_ERR_INVALID, "null field");
     if (n < 0) return fail(SP_ERR_INVALID, "negative step count");
     if (n == 0) return SP_OK;  // Convection.cpp:296: no step, output untouched
-    if ((rc = h->ensure_scratch(prec, 1))) return rc;
     const Geo& g = h->g[prec];
     cudaStream_t s = h->stream();
     int* err = h->err.as<int>();
@@ -423,6 +436,9 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
     if (!aligned16(in) && !tuned) t.no_small();
     const bool resident = rk && t.resident() && prec == 0 && cluster_supported(g, t.resident());
     const bool pairs = !resident && rk && prec == 0 && t.pairs() && pair_supported(h->g4);
+    const bool const_nu = h->P.nufreq == 0.;
+    const bool chunks = const_nu && n - 1 >= kChunk && !capturing(s);
+    if ((rc = h->ensure_scratch(prec, 1))) return rc;
     if (!(aligned16(in) && aligned16(out)) && tuned && !resident && !pairs && all_direct(t, rk)) {
         if ((rc = h->ensure_scratch(prec, 2))) return rc;  // copies in fields 3 and 4 of the 2-item scratch
         SP_CUDA(launch_periodicity(g, const_cast<void*>(in), 1, s));
@@ -431,7 +447,6 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
         SP_CUDA(cudaMemcpyAsync(out, h->sbuf(prec, 4, 1), g.total * g.es, cudaMemcpyDeviceToDevice, s));
         return SP_OK;
     }
-    const bool const_nu = h->P.nufreq == 0.;
     // Periodicity on the input, in place, as before the reference's first stencil
     // (the cluster-resident path writes the images of its input itself).
     if (!resident) SP_CUDA(launch_periodicity(g, const_cast<void*>(in), 1, s));
@@ -461,7 +476,7 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
         if ((rc = h->ensure_wide(1))) return rc;
         SP_CUDA(launch_widen(h->g4, h->wbuf(0, 1), g, in, 1, nullptr, 0, s));
         int i = 0;
-        if (const_nu && !capturing(s) && n - 1 >= kChunk) {
+        if (chunks) {
             GraphEntry* ge = nullptr;
             if ((rc = get_fused_graph(h, dt, computenu(h->P.nu0, h->P.nufreq, tStart), kChunk, &ge))) return rc;
             for (; n - 1 - i >= kChunk; i += kChunk) {  // kChunk is even: every chunk starts at wbuf(0)
@@ -478,29 +493,25 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
                                       last ? out : A, last ? g : h->g4, 1, nullptr, 0, s, err));
         }
     } else if (rk) {
+        void* const q = chunks && h->keeps_state(prec) ? h->state(prec) : out;  // the state between steps
         SP_CUDA(enqueue_rk4_step(g, prec, h->coef, dt, NuSrc{computenu(h->P.nu0, h->P.nufreq, tStart), nullptr}, in,
-                                 out, h->sbuf(prec, 0, 1), h->sbuf(prec, 1, 1), h->sbuf(prec, 2, 1), 1, nullptr, 0, t,
+                                 q, h->sbuf(prec, 0, 1), h->sbuf(prec, 1, 1), h->sbuf(prec, 2, 1), 1, nullptr, 0, t,
                                  s, err));
-        int i = 0;
-        int left = n - 1;
-        if (const_nu && !capturing(s)) {
-            const double nu = computenu(h->P.nu0, h->P.nufreq, tStart);
-            if (left >= kChunk) {
-                GraphEntry* ge = nullptr;
-                if ((rc = get_chunk_graph(h, prec, out, dt, nu, kChunk, &ge))) return rc;
-                while (left >= kChunk) {
-                    SP_CUDA(cudaGraphLaunch(ge->exec, s));
-                    add_launches(ge->nodes);
-                    left -= kChunk;
-                    i += kChunk;
-                }
+        int i = 1;
+        if (chunks) {
+            GraphEntry* ge = nullptr;
+            if ((rc = get_chunk_graph(h, prec, q, dt, computenu(h->P.nu0, h->P.nufreq, tStart), kChunk, &ge))) return rc;
+            for (; n - i >= kChunk; i += kChunk) {
+                SP_CUDA(cudaGraphLaunch(ge->exec, s));
+                add_launches(ge->nodes);
             }
         }
-        for (; left > 0; --left) {
-            const double tt = tStart + (++i) * dt;  // Convection.cpp:302
-            SP_CUDA(enqueue_rk4_step(g, prec, h->coef, dt, NuSrc{computenu(h->P.nu0, h->P.nufreq, tt), nullptr}, out,
-                                     out, h->sbuf(prec, 0, 1), h->sbuf(prec, 1, 1), h->sbuf(prec, 2, 1), 1, nullptr, 0,
-                                     t, s, err));
+        if (i == n && q != out) SP_CUDA(cudaMemcpyAsync(out, q, g.total * g.es, cudaMemcpyDeviceToDevice, s));
+        for (; i < n; ++i) {
+            const double tt = tStart + i * dt;  // Convection.cpp:302
+            SP_CUDA(enqueue_rk4_step(g, prec, h->coef, dt, NuSrc{computenu(h->P.nu0, h->P.nufreq, tt), nullptr}, q,
+                                     i + 1 < n ? q : out, h->sbuf(prec, 0, 1), h->sbuf(prec, 1, 1), h->sbuf(prec, 2, 1),
+                                     1, nullptr, 0, t, s, err));
         }
     } else {
         // Euler: one fused pass per step (out = in + dt R2(in)) needs distinct

@@ -156,3 +156,42 @@ def test_kernel_times_names_the_kernels_that_run(sp, n, tune):
     before = b.data.clone()
     assert len(c.kernel_times(a, 1e-5, reps=2)) == counts[1] - counts[0]
     assert bool((b.data == before).all())
+
+
+@pytest.mark.parametrize("n", [(48, 20, 24), (47, 20, 24), (2, 3, 5)])
+@pytest.mark.parametrize("prec", [0, 1], ids=["f64", "f32"])
+def test_runs_across_graph_chunks(sp, n, prec):
+    """Captured chunks of 50 steps, on the direct kernels (wrapping, with images) and the
+    TMA ring: out of place, in place and on fields the handle has not seen."""
+    c = conv_of(sp, n)
+    q0 = gaussian_noise(*n, seed=12)
+    for steps_ in (50, 51, 52, 101, 130):
+        c.set_tune(prec, 1, 4, 8, 1)
+        a, b = c.field(prec), c.field(prec)
+        c.upload(a, q0)
+        for _ in range(steps_):  # one at a time: no chunk
+            c.DoRK4(a, a, 0.0, 1e-4, 1)
+        c.Periodicity(a)
+        for tune in ((4, 8, 1), (8, 2, 0), (4, 1, 0)):
+            c.set_tune(prec, 1, *tune)
+            for inplace in (False, True, False):
+                x = c.field(prec)
+                y = x if inplace else c.field(prec)
+                c.upload(x, q0)
+                c.DoRK4(x, y, 0.0, 1e-4, steps_)
+                assert np.array_equal(c.download(y), c.download(a)), (steps_, tune, inplace)
+                assert halo_ok(c, y)
+
+
+@pytest.mark.parametrize("n", [(48, 20, 24), (17, 20, 24)])
+@pytest.mark.parametrize("prec", [0, 1], ids=["f64", "f32"])
+def test_euler_leaves_both_halos(sp, n, prec):
+    """Euler runs on the wrapping kernel write no images: the result's are made after."""
+    c = conv_of(sp, n)
+    for steps_ in (1, 2, 3):
+        for inplace in (False, True):
+            x = c.field(prec)
+            y = x if inplace else c.field(prec)
+            c.upload(x, gaussian_noise(*n, seed=13))
+            c.DoEuler(x, y, 0.0, 1e-4, steps_)
+            assert halo_ok(c, x) and halo_ok(c, y)
