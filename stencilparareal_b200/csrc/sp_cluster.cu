@@ -856,9 +856,9 @@ int default_cluster_mode(const Geo& g, int items) {
     return slabs < blocks ? 1 : 2;
 }
 
-cudaError_t prepare_cluster() {
+cudaError_t prepare_cluster(bool vary) {
     const cudaError_t e = prepare_cluster_kernels(false);
-    return e != cudaSuccess ? e : prepare_cluster_kernels(true);
+    return e != cudaSuccess || !vary ? e : prepare_cluster_kernels(true);
 }
 
 cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_t s, int* err) {

@@ -608,11 +608,11 @@ unsigned long long take_store_violations_pairs() {
     return v;
 }
 
-cudaError_t prepare_pairs() {
+cudaError_t prepare_pairs(bool per_item) {
     cudaError_t e = set_pair_attrs<0, 1>();
     if (e == cudaSuccess) e = set_pair_attrs<1, 1>();
-    if (e == cudaSuccess) e = set_pair_attrs<0, kItemWeights>();
-    if (e == cudaSuccess) e = set_pair_attrs<1, kItemWeights>();
+    if (e == cudaSuccess && per_item) e = set_pair_attrs<0, kItemWeights>();
+    if (e == cudaSuccess && per_item) e = set_pair_attrs<1, kItemWeights>();
     return e;
 }
 

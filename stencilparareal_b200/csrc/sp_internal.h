@@ -132,7 +132,7 @@ bool cluster_supported(const Geo& g, int mode = 1);
 // The mode for launches of `items` fields before tuning, on the current device (0:
 // other paths are faster, or the grid or device has no cluster layout).
 int default_cluster_mode(const Geo& g, int items);
-cudaError_t prepare_cluster();
+cudaError_t prepare_cluster(bool vary);
 cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_t s, int* err);
 constexpr int kClusterSmemMax = 227 * 1024;
 
@@ -179,7 +179,7 @@ cudaError_t launch_pair(const Geo& g4, const Geo& go, const PairLaunch& L, const
 // dst (geometry g4) <- interior of src (geometry gs), with g4.halo-deep images (FP64, items fields).
 cudaError_t launch_widen(const Geo& g4, void* dst, const Geo& gs, const void* src, int items, const int* item_lo,
                          int item_base, cudaStream_t s);
-cudaError_t prepare_pairs();
+cudaError_t prepare_pairs(bool per_item);
 // Stores counted outside their output allocation by the bounds-checked build
 // (stage kernels; pair and widening kernels; cluster kernels) since the previous
 // call; reset.
@@ -198,7 +198,10 @@ cudaError_t launch_field_to_dense(const Geo& g, const void* field, void* dense, 
 cudaError_t launch_convert(const Geo& gd, void* dst, const Geo& gs, const void* src, cudaStream_t s,
                            const int* item_lo = nullptr, int item = 0);
 // Sets the dynamic shared-memory limit of every TMA stage kernel on the current device.
-cudaError_t prepare_kernels();
+// Raises the kernels' shared-memory limits, which loads them (0.1-0.5 ms each, once per
+// process): those for one diffusivity per item or step only for handles that have
+// nu(t).
+cudaError_t prepare_kernels(bool per_item);
 // Parareal correction: Q = (gnew + f) - gold written to u_next (FP64, with images);
 // gold <- gnew; defect sums (sum (Q-u_old)^2, sum Q^2) atomically added to def[0..1].
 cudaError_t launch_update(const Geo& g64, const Geo& gc, const void* gnew, const double* f, void* gold,

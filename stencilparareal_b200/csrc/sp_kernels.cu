@@ -927,21 +927,23 @@ unsigned long long take_store_violations_stages() {
     return v;
 }
 
-cudaError_t prepare_kernels() {
+cudaError_t prepare_kernels(bool per_item) {
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
     chk(set_attr_op<double, OP_RK_S1>()); chk(set_attr_op<double, OP_RK_S2>());
     chk(set_attr_op<double, OP_RK_S3>()); chk(set_attr_op<double, OP_RK_S4>());
     chk(set_attr_op<double, OP_EULER>());
-    chk(set_attr_op<double, OP_RK_S1, kItemWeights>()); chk(set_attr_op<double, OP_RK_S2, kItemWeights>());
-    chk(set_attr_op<double, OP_RK_S3, kItemWeights>()); chk(set_attr_op<double, OP_RK_S4, kItemWeights>());
+    if (per_item) {
+        chk(set_attr_op<double, OP_RK_S1, kItemWeights>()); chk(set_attr_op<double, OP_RK_S2, kItemWeights>());
+        chk(set_attr_op<double, OP_RK_S3, kItemWeights>()); chk(set_attr_op<double, OP_RK_S4, kItemWeights>());
+    }
     chk(set_attr_op<double, OP_ADJ + 0>()); chk(set_attr_op<double, OP_ADJ + 1>());
     chk(set_attr_op<double, OP_ADJ + 2>()); chk(set_attr_op<double, OP_ADJ + 3>());
     chk(set_attr_op<float, OP_RK_S1>()); chk(set_attr_op<float, OP_RK_S2>());
     chk(set_attr_op<float, OP_RK_S3>()); chk(set_attr_op<float, OP_RK_S4>());
     chk(set_attr_op<float, OP_EULER>());
-    chk(prepare_pairs());
-    chk(prepare_cluster());
+    chk(prepare_pairs(per_item));
+    chk(prepare_cluster(per_item));
     return e;
 }
 

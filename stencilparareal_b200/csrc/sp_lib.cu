@@ -581,7 +581,7 @@ int sp_convection_create(const sp_params* p, int device, sp_convection** out) {
     SP_CUDA(cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking));
     if (h->err.alloc(64) != cudaSuccess) return fail(SP_ERR_NOMEM, "error word");
     if (h->red.alloc(64 * sizeof(double)) != cudaSuccess) return fail(SP_ERR_NOMEM, "reduction scratch");
-    SP_CUDA(prepare_kernels());
+    SP_CUDA(prepare_kernels(p->nufreq != 0.));
     *out = h.release();
     return SP_OK;
 }

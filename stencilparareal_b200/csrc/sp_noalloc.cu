@@ -71,7 +71,7 @@ cudaError_t device_setup(int dev, DeviceSetup** out) {
     void* q = nullptr;
     if ((e = cudaGetSymbolAddress(&p, g_scratch)) != cudaSuccess) return e;
     if ((e = cudaGetSymbolAddress(&q, g_err_word)) != cudaSuccess) return e;
-    if ((e = sp::prepare_kernels()) != cudaSuccess) return e;
+    if ((e = sp::prepare_kernels(false)) != cudaSuccess) return e;
     s.scratch = p;
     s.err = static_cast<int*>(q);
     s.done = true;
