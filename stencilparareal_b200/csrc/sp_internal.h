@@ -200,7 +200,7 @@ cudaError_t launch_convert(const Geo& gd, void* dst, const Geo& gs, const void* 
 // Sets the dynamic shared-memory limit of every TMA stage kernel on the current device.
 // Raises the kernels' shared-memory limits, which loads them (0.1-0.5 ms each, once per
 // process): those for one diffusivity per item or step only for handles that have
-// nu(t).
+// nu(t), the cluster kernels (prepare_cluster) only for grids they take.
 cudaError_t prepare_kernels(bool per_item);
 // Parareal correction: Q = (gnew + f) - gold written to u_next (FP64, with images);
 // gold <- gnew; defect sums (sum (Q-u_old)^2, sum Q^2) atomically added to def[0..1].

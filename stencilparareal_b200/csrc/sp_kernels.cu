@@ -943,7 +943,6 @@ cudaError_t prepare_kernels(bool per_item) {
     chk(set_attr_op<float, OP_RK_S3>()); chk(set_attr_op<float, OP_RK_S4>());
     chk(set_attr_op<float, OP_EULER>());
     chk(prepare_pairs(per_item));
-    chk(prepare_cluster(per_item));
     return e;
 }
 

@@ -582,6 +582,7 @@ int sp_convection_create(const sp_params* p, int device, sp_convection** out) {
     if (h->err.alloc(64) != cudaSuccess) return fail(SP_ERR_NOMEM, "error word");
     if (h->red.alloc(64 * sizeof(double)) != cudaSuccess) return fail(SP_ERR_NOMEM, "reduction scratch");
     SP_CUDA(prepare_kernels(p->nufreq != 0.));
+    if (cluster_supported(h->g[0], 1) || cluster_supported(h->g[0], 2)) SP_CUDA(prepare_cluster(p->nufreq != 0.));
     *out = h.release();
     return SP_OK;
 }
