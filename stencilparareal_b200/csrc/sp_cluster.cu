@@ -675,7 +675,9 @@ int resident_clusters(int C) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_rk4_cluster<2, 1, BANK>, &cfg) != cudaSuccess) {
+    // asked before the first handle is ready as well: without the attributes the answer is 0
+    if (set_attr_cluster(k_rk4_cluster<2, 1, BANK>) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, k_rk4_cluster<2, 1, BANK>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;  // asked again next time
     }

@@ -3,6 +3,10 @@ of a DoRK4 call in one launch, each field held in the shared memory of one
 thread-block cluster, split into z-slabs (tune kind 3) or into (y,z) blocks
 (kind 5).  They must give the four single-stage kernels' fields bit for bit
 (same operations, same order) and the oracle's to 1e-12."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -223,3 +227,34 @@ def test_every_form_leaves_both_halos_as_periodicity_does(sp, n, kind, nufreq):
         got.append((a.data.clone(), b.data.clone()))
     assert torch.equal(got[0][0], got[1][0])
     assert torch.equal(got[0][1], got[1][1])
+
+
+FIRST_HANDLE = r"""
+import sys
+sys.path[:0] = [{root!r}, {tests!r}]
+import stencilparareal_b200 as sp
+from ics import gaussian_noise
+n, P, steps = 24, 64, 200
+best = {{}}
+for kind in (3, 5):
+    c = sp.Convection(n, n, n, 1.0 / n, 0.01, 0.0, 1.0, 1.0, 1.0)
+    c.set_tune(sp.SP_F64, P, 0, 0, kind)
+    conf = sp.RuntimeConfiguration(timeSlices=P, nu0=0.01, gridSize=n, endTime=1e-5 * steps * P,
+                                   timeStepsFine=steps * P, timeStepsCoarse=P, kmax=1)
+    a, b = c.field(), c.field()
+    c.upload(a, gaussian_noise(n, seed=0))
+    par = sp.Parareal(c, a, b, 0.0, conf, coarse="rk4", coarse_precision="f32")
+    best[kind] = min(par.DoParallel()["seconds_fine"] for _ in range(6))
+print(best[3] / best[5])
+"""
+
+
+def test_first_handle_of_a_process_knows_how_many_clusters_fit(sp):
+    """The slabs' cluster size for a batch rests on how many clusters run at once, which is
+    asked while the process's first handle is made: 64 fields of 24^3 in clusters of six
+    CTAs take 0.83 of the blocks' time, in clusters of twelve 1.65."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    script = FIRST_HANDLE.format(root=root, tests=os.path.join(root, "tests"))
+    r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert float(r.stdout.split()[-1]) < 1.2
