@@ -960,12 +960,41 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
     SP_CUDA(cudaEventCreate(&e0));
     SP_CUDA(cudaEventCreate(&e1));
     Tune best = h->tune(precision, batch);
+    int* const err = h->err.as<int>();
+    const double nu0 = computenu(h->P.nu0, h->P.nufreq, 0.0);
+    // `k` steps on the stage kernels, in place on the first field
+    auto stage_steps = [&](const Tune& t, int k) {
+        cudaError_t x = cudaSuccess;
+        for (int i = 0; i < k && x == cudaSuccess; ++i)
+            x = enqueue_rk4_step(g, precision, h->coef, dtt, NuSrc{nu0, nullptr}, p, p, p + fb, p + 2 * fb, p + 3 * fb,
+                                 batch, nullptr, 0, t, s, err);
+        return x;
+    };
+    // the fastest of `reps` runs of fn, after one untimed
+    auto timed = [&](int reps, auto&& fn, float& ms) -> int {
+        int rc = fn();
+        for (int r = 0; r < reps && rc == SP_OK; ++r) {
+            cudaEventRecord(e0, s);
+            rc = fn();
+            cudaEventRecord(e1, s);
+            cudaEventSynchronize(e1);
+            float m = 0;
+            cudaEventElapsedTime(&m, e0, e1);
+            ms = std::min(ms, m);
+        }
+        return rc;
+    };
+    // A DoRK4 of one graph chunk of steps on tune t, as an untimed run has captured it
+    auto propagate = [&](const Tune& t, int n) -> int {
+        h->tunes[{precision, batch}] = t;
+        return do_prop(h, precision, true, p, p + fb, 0.0, dtt, n);
+    };
     std::vector<int> zcs = {1, 2, 3, 4, 8, 16, 32, 64};
     zcs.push_back(g.nk);
-    float op_ms[kNumOps], direct_ms[kNumOps];
-    Shape direct[kNumOps];  // the best direct shape of each stage
+    float op_ms[kNumOps], wrap_ms[kNumOps];
+    Shape chain[kNumOps];  // the best shape of each stage as a wrapping direct kernel
     for (auto& m : op_ms) m = 1e30f;
-    for (auto& m : direct_ms) m = 1e30f;
+    for (auto& m : wrap_ms) m = 1e30f;
     for (int op : {OP_RK_S1, OP_RK_S2, OP_RK_S3, OP_RK_S4, OP_EULER}) {
         StageLaunch L;
         L.op = op;
@@ -975,7 +1004,6 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
         L.nu = h->P.nu0;
         L.yin = p; L.q = p + fb; L.acc = p + 2 * fb; L.yout = p + 3 * fb;
         L.c_y = 1e-9; L.c_acc = 1e-9;
-        float best_ms = 1e30f;
         for (int kind = 1; kind >= 0; --kind)
             for (int ty : {4, 8, 16})
                 for (int zc : zcs) {
@@ -985,50 +1013,79 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
                     Shape sh;
                     sh.tma = kind; sh.ty = ty; sh.zchunk = zc;
                     t.set_all(sh);
-                    L.wrap = kind == 0 && wrap_supported(g);  // as in a step of direct kernels
-                    cudaError_t e = launch_stage(g, L, t, s, h->err.as<int>());
-                    if (e != cudaSuccess) { cudaGetLastError(); continue; }
-                    float ms = 1e30f;
-                    for (int r = 0; r < 3; ++r) {
-                        cudaEventRecord(e0, s);
-                        launch_stage(g, L, t, s, h->err.as<int>());
-                        cudaEventRecord(e1, s);
-                        cudaEventSynchronize(e1);
-                        float m = 0;
-                        cudaEventElapsedTime(&m, e0, e1);
-                        ms = std::min(ms, m);
+                    // a direct stage wraps where all of a step's stages are direct, and
+                    // writes images beside TMA stages
+                    for (int wrap = 0; wrap < (kind == 0 && wrap_supported(g) ? 2 : 1); ++wrap) {
+                        L.wrap = wrap;
+                        auto launch = [&]() { return launch_stage(g, L, t, s, err) == cudaSuccess ? SP_OK : SP_ERR_CUDA; };
+                        float ms = 1e30f;
+                        if (timed(3, launch, ms) != SP_OK) { cudaGetLastError(); continue; }
+                        if ((op == OP_EULER || !wrap) && ms < op_ms[op]) { op_ms[op] = ms; best.op[op] = sh; }
+                        if (wrap && ms < wrap_ms[op]) { wrap_ms[op] = ms; chain[op] = sh; }
                     }
-                    if (ms < best_ms) { best_ms = ms; best.op[op] = sh; }
-                    if (kind == 0 && ms < direct_ms[op]) { direct_ms[op] = ms; direct[op] = sh; }
                 }
-        op_ms[op] = best_ms;
     }
-    // RK4 steps whose four stages are all direct run as a chain without images, and
-    // overlap more than isolated timings show: they are taken unless those are more
-    // than 10 % worse than the best mixture's (128^3 FP64: chain 49 us per step, TMA 54),
-    // on the default's shape, measured in such chains, where that is direct (160^3
-    // FP32 50 us per step, with the isolated best of each stage 55-58)
-    float mixed = 0, chain = 0;
-    for (int op : {OP_RK_S1, OP_RK_S2, OP_RK_S3, OP_RK_S4}) {
-        mixed += op_ms[op];
-        chain += direct_ms[op];
-    }
-    const Shape dsh = default_stage_shape(g, batch);
-    if (wrap_supported(g) && chain < 1.1f * mixed)
-        for (int op : {OP_RK_S1, OP_RK_S2, OP_RK_S3, OP_RK_S4}) {
-            best.op[op] = dsh.tma ? direct[op] : dsh;
-            op_ms[op] = direct_ms[op];
+    // RK4 steps: the best shapes by themselves, a chain of wrapping direct stages on their
+    // best shapes, or the default's direct shape (160^3 FP32 50 us per step, with the
+    // isolated best of each stage 55-58; 95^3 FP64 24.0 / 27.2) -- by timing whole steps, since
+    // direct stages overlap more than isolated times show (128^3 FP64: chain 49 us, TMA
+    // 54)
+    {
+        const int ops[] = {OP_RK_S1, OP_RK_S2, OP_RK_S3, OP_RK_S4};
+        const Shape dsh = default_stage_shape(g, batch);
+        Tune cand[3] = {best, best, best};
+        float alone = 0, wrapped = 0;
+        for (int op : ops) {
+            cand[1].op[op] = chain[op];
+            cand[2].op[op] = dsh;
+            alone += op_ms[op];
+            wrapped += wrap_ms[op];
         }
+        const bool use[3] = {true, wrapped < 1.5f * alone, !dsh.tma};
+        float ms[3] = {1e30f, 1e30f, 1e30f};
+        SP_CUDA(fill_wave(p, 4 * fb, g.es, s));
+        for (int c = 0; c < 3 && (use[1] || use[2]) && rc == SP_OK; ++c) {
+            if (!use[c]) continue;
+            cand[c].fused = cand[c].cluster = 0;
+            cand[c].no_small();
+            h->drop_graphs();
+            rc = timed(5, [&]() -> int {
+                if (batch == 1) return propagate(cand[c], kChunk + 1);
+                const cudaError_t x = stage_steps(cand[c], 4);
+                return x == cudaSuccess ? SP_OK : fail(SP_ERR_CUDA, "tuning: %s", cudaGetErrorString(x));
+            }, ms[c]);
+        }
+        if (rc != SP_OK) {
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            h->drop_graphs();
+            return rc;
+        }
+        const int c = (int)(std::min_element(ms, ms + 3) - ms);
+        if (c)
+            for (int op : ops) best.op[op] = cand[c].op[op];
+    }
     // fused stage pairs (FP64): best shape per pair, then fused or single-stage
     // steps by timing whole steps of both paths
     best.fused = best.cluster = 0;
     best.no_small();
-    if (precision == SP_F64 && pair_supported(h->g4)) {
-        const Geo& g4 = h->g4;
-        const size_t wb = (size_t)batch * g4.total * g4.es;
-        DevBuf wbuf;
+    const Geo& g4 = h->g4;
+    const size_t wb = (size_t)batch * g4.total * g4.es;
+    DevBuf wbuf;
+    char* w = nullptr;
+    // `k` steps on the pairs, from the first wide field
+    auto pair_steps = [&](const Tune& t, int k) {
+        cudaError_t x = cudaSuccess;
+        for (int i = 0; i < k && x == cudaSuccess; ++i) {
+            char* Q = w + (size_t)(i % 2) * wb;
+            char* A = w + (size_t)((i + 1) % 2) * wb;
+            x = enqueue_pair_step(h, t, dtt, nu0, Q, A, w + 2 * wb, A, g4, batch, nullptr, 0, s, err);
+        }
+        return x;
+    };
+    if (precision == SP_F64 && pair_supported(g4)) {
         if (wbuf.alloc(3 * wb) == cudaSuccess) {
-            char* w = wbuf.as<char>();
+            w = wbuf.as<char>();
             float pair_ms[2] = {1e30f, 1e30f};
             float narrow_ms[2] = {1e30f, 1e30f};  // the best shape on 32 x 16 tiles
             Shape narrow[2];
@@ -1068,8 +1125,6 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
             alt.pair[1] = narrow[1];
             const bool try_narrow = narrow_ms[0] < 1e29f && narrow_ms[1] < 1e29f &&
                                     !(same_shape(alt.pair[0], best.pair[0]) && same_shape(alt.pair[1], best.pair[1]));
-            best.fused = (pair_ms[0] + pair_ms[1]) < (op_ms[OP_RK_S1] + op_ms[OP_RK_S2] + op_ms[OP_RK_S3] +
-                                                      op_ms[OP_RK_S4]) ? 1 : 0;
             if (batch == 1) {
                 // Single fields: decide by DoRK4 itself (one graph chunk of
                 // steps), where consecutive kernels overlap through programmatic
@@ -1080,20 +1135,10 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
                 for (int f = 0; f < (try_narrow ? 3 : 2) && rc == SP_OK; ++f) {
                     Tune tt = f == 2 ? alt : best;
                     tt.fused = f ? 1 : 0;
-                    h->tunes[{precision, batch}] = tt;
                     h->drop_graphs();
-                    rc = do_prop(h, precision, true, p, p + fb, 0.0, dtt, kChunk + 1);  // captures the graph
-                    if (rc == SP_OK)  // at the clocks the path sustains
-                        rc = sustain(s, [&]() { return do_prop(h, precision, true, p, p + fb, 0.0, dtt, kChunk + 1); });
-                    for (int r = 0; r < 3 && rc == SP_OK; ++r) {
-                        cudaEventRecord(e0, s);
-                        rc = do_prop(h, precision, true, p, p + fb, 0.0, dtt, kChunk + 1);
-                        cudaEventRecord(e1, s);
-                        cudaEventSynchronize(e1);
-                        float m = 0;
-                        cudaEventElapsedTime(&m, e0, e1);
-                        path_ms[f] = std::min(path_ms[f], m);
-                    }
+                    auto run = [&]() { return propagate(tt, kChunk + 1); };
+                    if ((rc = run()) == SP_OK) rc = sustain(s, run);  // at the clocks the path sustains
+                    if (rc == SP_OK) rc = timed(3, run, path_ms[f]);
                 }
                 if (rc != SP_OK) {
                     cudaEventDestroy(e0);
@@ -1112,28 +1157,10 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
                 // each path as the sweep launches them, after one untimed step.
                 SP_CUDA(fill_wave(p, 4 * fb, g.es, s));
                 SP_CUDA(fill_wave(w, 3 * wb, g4.es, s));
-                const double nu = computenu(h->P.nu0, h->P.nufreq, 0.0);
-                int* err = h->err.as<int>();
                 Tune ts = best;
                 ts.fused = 0;
-                auto stage_steps = [&](int k) {
-                    cudaError_t x = cudaSuccess;
-                    for (int i = 0; i < k && x == cudaSuccess; ++i)
-                        x = enqueue_rk4_step(g, precision, h->coef, dtt, NuSrc{nu, nullptr}, p, p, p + fb,
-                                             p + 2 * fb, p + 3 * fb, batch, nullptr, 0, ts, s, err);
-                    return x;
-                };
-                auto pair_steps = [&](const Tune& pt, int k) {
-                    cudaError_t x = cudaSuccess;
-                    for (int i = 0; i < k && x == cudaSuccess; ++i) {
-                        char* Q = w + (size_t)(i % 2) * wb;
-                        char* A = w + (size_t)((i + 1) % 2) * wb;
-                        x = enqueue_pair_step(h, pt, dtt, nu, Q, A, w + 2 * wb, A, h->g4, batch, nullptr, 0, s, err);
-                    }
-                    return x;
-                };
                 auto path_steps = [&](int f, int k) {
-                    return f == 0 ? stage_steps(k) : pair_steps(f == 2 ? alt : best, k);
+                    return f == 0 ? stage_steps(ts, k) : pair_steps(f == 2 ? alt : best, k);
                 };
                 float path_ms[3] = {1e30f, 1e30f, 1e30f};  // stages, best pairs, pairs on 32 x 16 tiles
                 cudaError_t x = cudaSuccess;
@@ -1172,44 +1199,31 @@ extern "C" int sp_autotune(sp_convection* h, int precision, int batch) {
     }
     // small fields: the cluster-resident paths (z-slabs, (y,z) blocks) against
     // the best of the above, timed as they are used (a DoRK4 of a graph chunk of
-    // steps for one field; as many batched steps for a batch: a cluster launch loads
-    // and stores its fields once, which over four steps hid its advantage)
+    // steps for one field; as many batched steps for a batch, of pairs where those
+    // were chosen: a cluster launch loads and stores its fields once, which over
+    // four steps hid its advantage)
     if (precision == SP_F64 && (cluster_supported(g, 1) || cluster_supported(g, 2))) {
-        int* err = h->err.as<int>();
         float path_ms[3] = {1e30f, 1e30f, 1e30f};
         SP_CUDA(fill_wave(p, 5 * fb, g.es, s));
+        if (w) SP_CUDA(fill_wave(w, 3 * wb, g4.es, s));
         for (int c = 0; c < 3 && rc == SP_OK; ++c) {
             if (c && !cluster_supported(g, c)) continue;
             Tune tt = best;
             tt.cluster = c;
-            h->tunes[{precision, batch}] = tt;
             h->drop_graphs();
-            auto run = [&]() -> int {
-                if (batch == 1) return do_prop(h, precision, true, p, p + fb, 0.0, dtt, kChunk + 1);
-                const double nu = computenu(h->P.nu0, h->P.nufreq, 0.0);
-                cudaError_t x = cudaSuccess;
+            rc = timed(3, [&]() -> int {
+                if (batch == 1) return propagate(tt, kChunk + 1);
+                cudaError_t x;
                 if (c) {
                     ClusterLaunch L;
                     L.mode = c;
-                    L.in = p; L.out = p; L.items = batch; L.nsteps = kChunk; L.dt = dtt; L.nu = &nu; L.coef = h->coef;
+                    L.in = p; L.out = p; L.items = batch; L.nsteps = kChunk; L.dt = dtt; L.nu = &nu0; L.coef = h->coef;
                     x = launch_rk4_cluster(g, L, s, err);
                 } else {
-                    for (int i = 0; i < kChunk && x == cudaSuccess; ++i)
-                        x = enqueue_rk4_step(g, precision, h->coef, dtt, NuSrc{nu, nullptr}, p, p, p + fb, p + 2 * fb,
-                                             p + 3 * fb, batch, nullptr, 0, tt, s, err);
+                    x = tt.pairs() ? pair_steps(tt, kChunk) : stage_steps(tt, kChunk);
                 }
                 return x == cudaSuccess ? SP_OK : fail(SP_ERR_CUDA, "tuning: %s", cudaGetErrorString(x));
-            };
-            rc = run();  // captures the graphs / warms up
-            for (int r = 0; r < 3 && rc == SP_OK; ++r) {
-                cudaEventRecord(e0, s);
-                rc = run();
-                cudaEventRecord(e1, s);
-                cudaEventSynchronize(e1);
-                float m = 0;
-                cudaEventElapsedTime(&m, e0, e1);
-                path_ms[c] = std::min(path_ms[c], m);
-            }
+            }, path_ms[c]);
             if (rc != SP_OK && c) {
                 // a cluster launch can be refused (cluster shape not schedulable): keep the other paths
                 cudaGetLastError();
