@@ -148,3 +148,57 @@ def test_cluster_stores_are_checked(checked_lib, shrink):
     assert r.returncode == 0, r.stderr[-2000:]
     out = json.loads(r.stdout.strip().splitlines()[-1])
     assert out["checked"] == 1 and (out["count"] > 0) == bool(shrink)
+
+
+SHAPES_SCRIPT = r"""
+import ctypes as C, json, sys
+sys.path.insert(0, {root!r}); sys.path.insert(0, {tests!r})
+import numpy as np
+import stencilparareal_b200 as sp
+from stencilparareal_b200.adjoint import misfit_gradient
+from ics import gaussian_noise
+L = sp._lib
+TUNES = [(4, 8, 1), (8, 3, 1), (16, 5, 1), (4, 1, 0), (8, 2, 0), (4, 5, 0)]
+# even and odd widths, rows beside a tile's, widths beside a TMA tile's
+for n in ((12, 12, 12), (13, 9, 7), (66, 17, 6), (2, 3, 5)):
+    conv = sp.Convection(*n, 1.0 / 12, 0.05, 0.0, 0.7, -0.4, 0.3)
+    f0, ft = conv.field(), conv.field()
+    conv.upload(f0, gaussian_noise(*n, seed=3, amp=1e-2))
+    conv.upload(ft, gaussian_noise(*n, seed=4, amp=1e-2))
+    for tune in TUNES:
+        conv.set_tune(sp.SP_F64, 1, *tune)
+        misfit_gradient(conv, f0, ft, 0.0, 2e-3, 6, checkpoint_every=2)
+for n in ((128, 5, 6), (132, 6, 7), (17, 19, 23), (4, 4, 4), (5, 130, 9)):
+    conv = sp.Convection(*n, 1.0 / n[0], 0.02, 0.0, 1.0, -0.5, 0.25)
+    gi, go = conv.field(sp.SP_F32), conv.field(sp.SP_F32)
+    conv.upload(gi, gaussian_noise(*n, seed=1))
+    for tune in TUNES:
+        conv.set_tune(sp.SP_F32, 1, *tune)
+        conv.DoRK4(gi, go, 0.0, 1e-4, 2)
+        conv.DoEuler(gi, go, 0.0, 1e-4, 2)
+# one diffusivity per slice, more slices than one launch takes
+for n in (10, 11):
+    P = 35
+    for tune in TUNES + [(8, 3, 2), (16, 0, 4)]:
+        conv = sp.Convection(n, n, n, 1.0 / n, 0.05, 20.0, 1.0, 0.5, -0.25)
+        conv.set_tune(sp.SP_F64, P, *tune)
+        conf = sp.RuntimeConfiguration(timeSlices=P, nu0=0.05, nufreq=20.0, gridSize=n, endTime=0.01, timeStepsFine=2 * P,
+                                       timeStepsCoarse=P, kmax=2)
+        fin, fsol = conv.field(), conv.field()
+        conv.upload(fin, gaussian_noise(n, seed=2))
+        sp.Parareal(conv, fin, fsol, 0.0, conf, coarse="rk4", coarse_precision="f32").DoParallel()
+chk, cnt = C.c_int(), C.c_longlong()
+L.check(L.lib().sp_store_violations(C.byref(chk), C.byref(cnt)))
+print(json.dumps({{"checked": chk.value, "count": cnt.value}}))
+"""
+
+
+def test_explicit_shapes_store_inside_their_allocations(checked_lib):
+    """Adjoint stages, FP32 stages and slices with a diffusivity of their own on TMA and
+    direct shapes set explicitly: what these sizes run by default is one of them."""
+    script = SHAPES_SCRIPT.format(root=ROOT, tests=os.path.join(ROOT, "tests"))
+    r = subprocess.run([sys.executable, "-c", script], env=dict(os.environ, STENCILPARAREAL_LIB=checked_lib),
+                       capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    out = json.loads(r.stdout.strip().splitlines()[-1])
+    assert out["checked"] == 1 and out["count"] == 0

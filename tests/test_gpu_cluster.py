@@ -258,3 +258,18 @@ def test_first_handle_of_a_process_knows_how_many_clusters_fit(sp):
     r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     assert float(r.stdout.split()[-1]) < 1.2
+
+
+@pytest.mark.parametrize("n,nufreq,in_place", [((22, 26, 30), 30.0, False), ((32, 32, 32), 30.0, True),
+                                               ((36, 36, 36), 0.0, False), ((16, 16, 16), 0.0, True)])
+def test_default_path_leaves_the_result_with_its_halo(sp, n, nufreq, in_place):
+    """An untuned handle over several launches (270 steps): the result's halo before any
+    Periodicity is the one Periodicity makes."""
+    c = _conv(sp, n, nufreq=nufreq)
+    a = c.field()
+    b = a if in_place else c.field()
+    c.upload(a, gaussian_noise(*n, seed=9))
+    c.DoRK4(a, b, 0.1, 1e-5, 270)
+    got = b.data.clone()
+    c.Periodicity(b)
+    assert torch.equal(got, b.data)
