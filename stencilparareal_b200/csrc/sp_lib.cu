@@ -118,8 +118,8 @@ struct sp_convection {
     Geo g4;            // FP64 with 4-cell halos: internal fields of the fused stage pairs
     Coef coef;
     cudaStream_t own = nullptr, user = nullptr;
-    DevBuf scratch[2];  // per precision: ya, yb, acc (x batch) for DoRK4 / Euler ping-pong
-    int scratch_items[2] = {0, 0};
+    DevBuf scratch[2];  // per precision: ya, yb, acc and the state between steps (see keeps_state)
+    DevBuf copies[2];   // per precision: an input and an output field (host buffers, unaligned fields)
     DevBuf wide;        // fused-pair fields (geometry g4): two step-start/accumulator fields and y2 (x batch)
     int wide_items = 0;
     DevBuf err;         // device error word
@@ -175,16 +175,23 @@ struct sp_convection {
     // was seen.  Larger fields take longer than that over one step, and the work field
     // would be felt.
     bool keeps_state(int prec) const { return (size_t)g[prec].total * g[prec].es <= (size_t)128 << 20; }
-    void* state(int prec) const { return sbuf(prec, 3 * scratch_items[prec], 1); }
-    int ensure_scratch(int prec, int items) {
-        if (scratch_items[prec] >= items) return SP_OK;
-        drop_graphs();  // captured graphs hold the old scratch addresses
-        const size_t n = ((size_t)3 * items + (keeps_state(prec) ? 1 : 0)) * g[prec].total * g[prec].es;
-        scratch_items[prec] = 0;  // a failing allocation leaves none
-        cudaError_t e = scratch[prec].alloc(n);
+    void* state(int prec) const { return sbuf(prec, 3); }
+    // Work fields, allocated once and never moved: a graph that a caller captured a call
+    // into holds their addresses.
+    int ensure_scratch(int prec) {
+        const size_t n = (size_t)(keeps_state(prec) ? 4 : 3) * g[prec].total * g[prec].es;
+        const cudaError_t e = scratch[prec].alloc(n);
         if (e != cudaSuccess) return fail(SP_ERR_NOMEM, "scratch allocation of %zu bytes: %s", n, cudaGetErrorString(e));
-        scratch_items[prec] = items;
         return SP_OK;
+    }
+    int ensure_copies(int prec) {
+        const size_t n = (size_t)2 * g[prec].total * g[prec].es;
+        const cudaError_t e = copies[prec].alloc(n);
+        if (e != cudaSuccess) return fail(SP_ERR_NOMEM, "two fields of %zu bytes: %s", n, cudaGetErrorString(e));
+        return SP_OK;
+    }
+    void* copy(int prec, int which) const {
+        return static_cast<char*>(copies[prec].p) + (size_t)which * g[prec].total * g[prec].es;
     }
     int ensure_wide(int items) {
         if (wide_items >= items) return SP_OK;
@@ -200,8 +207,8 @@ struct sp_convection {
     void* wbuf(int which, int items) const {
         return static_cast<char*>(wide.p) + (size_t)which * items * g4.total * g4.es;
     }
-    void* sbuf(int prec, int which, int items) const {
-        return static_cast<char*>(scratch[prec].p) + (size_t)which * items * g[prec].total * g[prec].es;
+    void* sbuf(int prec, int which) const {
+        return static_cast<char*>(scratch[prec].p) + (size_t)which * g[prec].total * g[prec].es;
     }
 };
 
@@ -300,7 +307,7 @@ int get_chunk_graph(sp_convection* h, int prec, void* field, double dt, double n
             if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
         h->graphs.clear();
     }
-    int rc = h->ensure_scratch(prec, 1);
+    int rc = h->ensure_scratch(prec);
     if (rc) return rc;
     const Tune t = h->tune(prec, 1);
     cudaStream_t s = h->stream();
@@ -308,8 +315,8 @@ int get_chunk_graph(sp_convection* h, int prec, void* field, double dt, double n
     cudaError_t e = cudaSuccess;
     const long long before = launches();
     for (int i = 0; i < n && e == cudaSuccess; ++i)
-        e = enqueue_rk4_step(h->g[prec], prec, h->coef, dt, NuSrc{nu, nullptr}, field, field, h->sbuf(prec, 0, 1),
-                             h->sbuf(prec, 1, 1), h->sbuf(prec, 2, 1), 1, nullptr, 0, t, s, h->err.as<int>());
+        e = enqueue_rk4_step(h->g[prec], prec, h->coef, dt, NuSrc{nu, nullptr}, field, field, h->sbuf(prec, 0),
+                             h->sbuf(prec, 1), h->sbuf(prec, 2), 1, nullptr, 0, t, s, h->err.as<int>());
     const long long nodes = launches() - before;
     add_launches(-nodes);  // captured, not launched
     cudaGraph_t graph = nullptr;
@@ -438,13 +445,15 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
     const bool pairs = !resident && rk && prec == 0 && t.pairs() && pair_supported(h->g4);
     const bool const_nu = h->P.nufreq == 0.;
     const bool chunks = const_nu && n - 1 >= kChunk && !capturing(s);
-    if ((rc = h->ensure_scratch(prec, 1))) return rc;
+    if ((rc = h->ensure_scratch(prec))) return rc;
     if (!(aligned16(in) && aligned16(out)) && tuned && !resident && !pairs && all_direct(t, rk)) {
-        if ((rc = h->ensure_scratch(prec, 2))) return rc;  // copies in fields 3 and 4 of the 2-item scratch
+        if ((rc = h->ensure_copies(prec))) return rc;
+        void* const ci = h->copy(prec, 0);
+        void* const co = h->copy(prec, 1);
         SP_CUDA(launch_periodicity(g, const_cast<void*>(in), 1, s));
-        SP_CUDA(cudaMemcpyAsync(h->sbuf(prec, 3, 1), in, g.total * g.es, cudaMemcpyDeviceToDevice, s));
-        if ((rc = do_prop(h, prec, rk, h->sbuf(prec, 3, 1), h->sbuf(prec, 4, 1), tStart, dt, n))) return rc;
-        SP_CUDA(cudaMemcpyAsync(out, h->sbuf(prec, 4, 1), g.total * g.es, cudaMemcpyDeviceToDevice, s));
+        SP_CUDA(cudaMemcpyAsync(ci, in, g.total * g.es, cudaMemcpyDeviceToDevice, s));
+        if ((rc = do_prop(h, prec, rk, ci, co, tStart, dt, n))) return rc;
+        SP_CUDA(cudaMemcpyAsync(out, co, g.total * g.es, cudaMemcpyDeviceToDevice, s));
         return SP_OK;
     }
     // Periodicity on the input, in place, as before the reference's first stencil
@@ -495,7 +504,7 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
     } else if (rk) {
         void* const q = chunks && h->keeps_state(prec) ? h->state(prec) : out;  // the state between steps
         SP_CUDA(enqueue_rk4_step(g, prec, h->coef, dt, NuSrc{computenu(h->P.nu0, h->P.nufreq, tStart), nullptr}, in,
-                                 q, h->sbuf(prec, 0, 1), h->sbuf(prec, 1, 1), h->sbuf(prec, 2, 1), 1, nullptr, 0, t,
+                                 q, h->sbuf(prec, 0), h->sbuf(prec, 1), h->sbuf(prec, 2), 1, nullptr, 0, t,
                                  s, err));
         int i = 1;
         if (chunks) {
@@ -510,13 +519,13 @@ int do_prop(sp_convection* h, int prec, bool rk, const void* in, void* out, doub
         for (; i < n; ++i) {
             const double tt = tStart + i * dt;  // Convection.cpp:302
             SP_CUDA(enqueue_rk4_step(g, prec, h->coef, dt, NuSrc{computenu(h->P.nu0, h->P.nufreq, tt), nullptr}, q,
-                                     i + 1 < n ? q : out, h->sbuf(prec, 0, 1), h->sbuf(prec, 1, 1), h->sbuf(prec, 2, 1),
+                                     i + 1 < n ? q : out, h->sbuf(prec, 0), h->sbuf(prec, 1), h->sbuf(prec, 2),
                                      1, nullptr, 0, t, s, err));
         }
     } else {
         // Euler: one fused pass per step (out = in + dt R2(in)) needs distinct
         // input and output, so steps alternate between `out` and scratch.
-        void* tmp = h->sbuf(prec, 0, 1);
+        void* tmp = h->sbuf(prec, 0);
         const void* src = in;
         for (int i = 0; i < n; ++i) {
             const double tt = i == 0 ? tStart : tStart + i * dt;
@@ -761,10 +770,10 @@ int sp_do_rk4_host(sp_convection* h, const double* in_host, double* out_host, do
     if (rc) return rc;
     if (!in_host || !out_host) return fail(SP_ERR_INVALID, "null host buffer");
     if (timesteps < 0) return fail(SP_ERR_INVALID, "negative step count");
-    if ((rc = h->ensure_scratch(0, 2))) return rc;  // fields 3 and 4 of the 2-item scratch hold in/out
+    if ((rc = h->ensure_scratch(0)) || (rc = h->ensure_copies(0))) return rc;
     const Geo& g = h->g[0];
-    double* f_in = static_cast<double*>(h->sbuf(0, 3, 1));
-    double* f_out = static_cast<double*>(h->sbuf(0, 4, 1));
+    double* f_in = static_cast<double*>(h->copy(0, 0));
+    double* f_out = static_cast<double*>(h->copy(0, 1));
     if ((rc = sp_field_import(h, in_host, f_in, SP_F64, 1))) return rc;
     if (timesteps == 0) {
         SP_CUDA(cudaMemcpyAsync(f_out, f_in, g.total * g.es, cudaMemcpyDeviceToDevice, h->stream()));
@@ -838,7 +847,7 @@ extern "C" int sp_kernel_times(sp_convection* h, const double* field, double dt,
     const bool fused = path == 2 || (path == 0 && (t.resident() ? t.fused : t.pairs()) && pair_supported(h->g4));
     if (fused) {
         if ((rc = h->ensure_wide(1))) return rc;
-    } else if ((rc = h->ensure_scratch(0, 2))) {  // fields 0, 3, 4, 5 of the 2-item scratch
+    } else if ((rc = h->ensure_scratch(0)) || (rc = h->ensure_copies(0))) {
         return rc;
     }
     // All launches are enqueued before one synchronisation, so that the GPU
@@ -867,10 +876,10 @@ extern "C" int sp_kernel_times(sp_convection* h, const double* field, double dt,
             cudaEventRecord(ev[(size_t)r * 2 + 2], s);
         }
     } else {
-        void* q = h->sbuf(0, 3, 1);
-        void* ya = h->sbuf(0, 4, 1);
-        void* yb = h->sbuf(0, 5, 1);
-        void* ac = h->sbuf(0, 0, 1);
+        void* q = h->copy(0, 0);
+        void* ya = h->sbuf(0, 0);
+        void* yb = h->sbuf(0, 1);
+        void* ac = h->sbuf(0, 2);
         if (e == cudaSuccess) e = cudaMemcpyAsync(q, field, g.total * g.es, cudaMemcpyDeviceToDevice, s);
         StageLaunch L;
         L.prec = 0; L.items = 1; L.nu = nu; L.coef = h->coef;
@@ -1856,7 +1865,7 @@ int sp_parareal_do_parallel(sp_parareal* pr, const double* initial, double* solu
     const int P = pr->P;
     const Geo& g = pr->g64;
     const int cp = pr->cprec;
-    if ((rc = h->ensure_scratch(cp, 1))) return rc;
+    if ((rc = h->ensure_scratch(cp))) return rc;
     if (rep) {
         std::memset(rep, 0, sizeof *rep);
         rep->tsFine = pr->tsF; rep->tsCoarse = pr->tsC;
@@ -2289,7 +2298,7 @@ extern "C" int sp_parareal_batch_run(sp_parareal_batch* b, const double* const* 
     for (int i = 0; i < n; ++i) {
         sp_parareal* pr = b->ins[i];
         if (!initial[i] || !solution[i]) return fail(SP_ERR_INVALID, "null field of instance %d", i);
-        int rc = pr->prop->ensure_scratch(pr->cprec, 1);
+        int rc = pr->prop->ensure_scratch(pr->cprec);
         if (rc) return rc;
         if (reports) {
             std::memset(&reports[i], 0, sizeof reports[i]);
@@ -2452,7 +2461,7 @@ extern "C" int sp_parareal_window_begin(sp_parareal* pr, const double* initial) 
     int rc = check_handle(pr->prop);
     if (rc) return rc;
     cudaStream_t s = pr->prop->stream();
-    if ((rc = pr->prop->ensure_scratch(pr->cprec, 1))) return rc;
+    if ((rc = pr->prop->ensure_scratch(pr->cprec))) return rc;
     if ((rc = window_graphs(pr))) return rc;
     return enqueue_predictor(pr, initial, s);
 }
