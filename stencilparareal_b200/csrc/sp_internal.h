@@ -99,6 +99,7 @@ struct StageLaunch {
     double sigma = 1;                // mu_s = sigma * (stencil input)
     double dnu = 1;                  // d nu / d nu0
     bool wrap = false;               // wrapping direct kernel: `yin` needs no images, `yout` gets none
+    bool drain = false;              // direct kernels: start once the kernel before has left the SMs
     int adj_first = 0;               // 1: lam_acc = lam + ybar (first adjoint stage of a step)
 };
 

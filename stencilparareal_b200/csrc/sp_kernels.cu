@@ -812,16 +812,17 @@ cudaError_t launch_direct_T(const Geo& g, const StageLaunch& L, KArgs<T> a, cons
     if (chunks > 0x7fffffffLL || grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
     Weights<T, NW> wt;
     fill_weights(wt, L.coef, L.nu, L.nu_items, L.items);
+    auto run = [&](auto k) { return launch_in_stream(!L.drain, k, grid, dim3(threads), 0, s, a, wt); };
     if (L.wrap) {
         constexpr int ZMAX = OpTraits<OP>::adjoint ? 2 : 4;  // (adjoint stages: 100 registers with two planes)
         switch (std::min(t.zchunk, ZMAX)) {
-            case 1: return launch_pdl(k_stage_wrap<T, OP, NW, 1>, grid, dim3(threads), 0, s, a, wt);
-            case 2: return launch_pdl(k_stage_wrap<T, OP, NW, 2>, grid, dim3(threads), 0, s, a, wt);
-            case 3: return launch_pdl(k_stage_wrap<T, OP, NW, std::min(3, ZMAX)>, grid, dim3(threads), 0, s, a, wt);
-            default: return launch_pdl(k_stage_wrap<T, OP, NW, ZMAX>, grid, dim3(threads), 0, s, a, wt);
+            case 1: return run(k_stage_wrap<T, OP, NW, 1>);
+            case 2: return run(k_stage_wrap<T, OP, NW, 2>);
+            case 3: return run(k_stage_wrap<T, OP, NW, std::min(3, ZMAX)>);
+            default: return run(k_stage_wrap<T, OP, NW, ZMAX>);
         }
     }
-    return launch_pdl(k_stage_direct<T, OP, NW>, grid, dim3(threads), 0, s, a, wt);
+    return run(k_stage_direct<T, OP, NW>);
 }
 
 template <typename T, int OP, int TY, int NS, int NP>

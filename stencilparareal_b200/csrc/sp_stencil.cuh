@@ -95,7 +95,8 @@ __device__ __forceinline__ T add_third(T y, T q, T base) {
 // this way call pdl_trigger/pdl_wait), so that in a stream or a captured graph the
 // next kernel's CTAs start while this one's last CTAs finish.
 template <typename... KP, typename... A>
-cudaError_t launch_pdl(void (*k)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+cudaError_t launch_in_stream(bool overlap, void (*k)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                             A&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -103,10 +104,14 @@ cudaError_t launch_pdl(void (*k)(KP...), dim3 grid, dim3 block, size_t smem, cud
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+template <typename... KP, typename... A>
+cudaError_t launch_pdl(void (*k)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    return launch_in_stream(true, k, grid, block, smem, s, std::forward<A>(args)...);
 }
 
 // Byte range of `items` fields of geometry g from `base`: the allocation a
