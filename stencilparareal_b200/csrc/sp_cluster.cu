@@ -689,8 +689,9 @@ int resident_clusters(int C) {
 // `cells` cells and receive `halo` values per stage; a halo value costs about half
 // the work of a cell.  Fitted to 16^3 ... 40^3 (est. / measured): slabs 16^3 2.1 / 2.2,
 // 24^3 3.6 / 3.6, 32^3 5.7 / 6.3, 36^3 8.4 / 9.3, 40^3 12.0 / 13.1; blocks 16^3 1.5 /
-// 1.6, 32^3 4.5 / 4.5; 16 fields of 32^3 in blocks (3 waves) 13.4 / 14.1.
+// 1.6, 32^3 4.5 / 4.4; 16 fields of 32^3 in blocks (3 waves) 13.4 / 13.0.
 double cluster_us(int C, int items, double cells, double halo) {
+    if (items == 0) return 0.;  // only whether a layout exists is asked: not of the device
     const int at_once = resident_clusters(C);
     if (!at_once) return 1e30;
     return (double)((items + at_once - 1) / at_once) * (0.95 + 1.15e-3 * (cells + 0.5 * halo));
@@ -698,8 +699,8 @@ double cluster_us(int C, int items, double cells, double halo) {
 
 // Planes per CTA for a grid and batch: the NZ in {2, 3, 4}, with a cluster of at
 // most 16 CTAs whose buffers fit, of the least estimated time; 0 when the grid is
-// not supported.
-int cluster_nz(const Geo& g, int items = 1, double* us = nullptr) {
+// not supported.  (items 0: any of them, the first.)
+int cluster_nz(const Geo& g, int items, double* us = nullptr) {
     if (g.es != 8 || g.ni % 2 != 0 || g.ni < 4 || g.nj < 4 || g.nk < 4) return 0;
     if ((long long)(g.ni / 2) * g.nj > 2LL * kClusterThreads) return 0;
     int best = 0;
@@ -747,15 +748,15 @@ size_t cluster2d_smem(int ni, int by, int bz) {
 // (y,z) blocks for a grid and batch: cy, cz >= 2 with C = cy * cz <= 16, blocks
 // of at least 2 rows and 2 planes whose two buffers fit, and a thread form
 // (below).  Among those the one with the least estimated time, x 1.6 for the
-// spilling two-unit form; ties go to fewer units per thread.  cy = 0 when the
-// grid has no such blocks.
+// spilling two-unit form (40^3 on blocks then 11.3 us, 12.0 measured); ties go to fewer
+// units per thread.  cy = 0 when the grid has no such blocks.  (items 0: any of them.)
 struct Blocks2d {
     int cy = 0, cz = 0, zt = 0, upt = 0, nt = 0;
     double us = 0;
 };
 Blocks2d blocks_2d(const Geo& g, int items) {
     Blocks2d best;
-    if (g.es != 8 || g.ni % 2 != 0 || g.ni < 4 || g.nj < 4 || g.nk < 4 || items < 1) return best;
+    if (g.es != 8 || g.ni % 2 != 0 || g.ni < 4 || g.nj < 4 || g.nk < 4) return best;
     for (int cy = 2; cy <= 8; ++cy)
         for (int cz = 2; cy * cz <= 16; ++cz) {
             if (g.nj % cy != 0 || g.nk % cz != 0) continue;
@@ -842,12 +843,12 @@ unsigned long long take_store_violations_cluster() {
 }
 
 bool cluster_supported(const Geo& g, int mode) {
-    return mode == 2 ? blocks_2d(g, 1).cy != 0 : cluster_nz(g) != 0;
+    return mode == 2 ? blocks_2d(g, 0).cy != 0 : cluster_nz(g, 0) != 0;
 }
 
 // Against the direct stage kernels, whose step takes about 9.5 us (four launches) +
-// 31 us per 1M cells: 32^3 10.7 us (cluster 4.5), 36^3 12.8 (9.3), 40^3 12.7 (13.1); 8
-// fields of 32^3 13.5 (9.4), 40 of them 48 (26), 8 of 40^3 27 (13.6).
+// 31 us per 1M cells: 32^3 10.7 us (cluster 4.4), 36^3 12.8 (9.1), 40^3 12.7 (12.0 on blocks,
+// 12.9 on slabs); 8 fields of 32^3 13.5 (8.6), 40 of them 48 (26), 8 of 40^3 27 (13.1).
 int default_cluster_mode(const Geo& g, int items) {
     double slabs = 1e30;
     if (!cluster_nz(g, items, &slabs)) slabs = 1e30;
@@ -864,9 +865,10 @@ cudaError_t prepare_cluster(bool vary) {
 }
 
 cudaError_t launch_rk4_cluster(const Geo& g, const ClusterLaunch& L, cudaStream_t s, int* err) {
+    if (L.nsteps < 1 || L.items < 1) return cudaErrorInvalidValue;
     const int nz = L.mode == 2 ? 0 : cluster_nz(g, L.items);
     const Blocks2d b2 = L.mode == 2 ? blocks_2d(g, L.items) : Blocks2d{};
-    if ((L.mode == 2 ? !b2.cy : !nz) || L.nsteps < 1 || L.items < 1) return cudaErrorInvalidValue;
+    if (L.mode == 2 ? !b2.cy : !nz) return cudaErrorInvalidValue;
     if (!L.nutab && (L.nu_count < 1 || L.nu_count > kClusterNuSteps || (L.nu_count > 1 && L.nu_count < L.nsteps)))
         return cudaErrorInvalidValue;
     if (!aligned16(L.in) || !aligned16(L.out)) return cudaErrorInvalidValue;
