@@ -17,9 +17,12 @@
  * fastest, like the reference's CUDA ConvectionField (Convection.h:13-17:
  * halo 2 in i, j and k; KJI order; i padded for alignment).  sp_field_layout()
  * gives the exact geometry: element (i,j,k), -2 <= i < ni+2 (same for j, k),
- * lives at  origin + k*plane + j*px + i.  Every kernel of this library that
- * writes a field also writes the periodic images of its boundary cells, so a
- * field produced by the library always has a valid halo.  A field written by
+ * lives at  origin + k*plane + j*px + i.  A field handed out by the library always
+ * has a valid halo (the kernels write the periodic images of boundary cells, or a last
+ * launch does).  Fields should start on a 16-byte boundary, as device allocations do: the
+ * kernels access them in 16-byte chunks, and a call refuses others, except as input of an
+ * sp_do_rk4 that runs on the fused pairs (without a tune: any) and where a tune forces
+ * the direct kernels, which go through aligned copies.  A field written by
  * the caller needs sp_periodicity_apply() (or sp_field_import(), which fills
  * the halo) -- exactly as the reference refreshes the input halo in place
  * before every stencil (Convection.cpp:328-334, Periodicity.h:60-66).
@@ -278,7 +281,8 @@ long long sp_launch_count(void);
  * grid badly) on the stage kernels (ops 0..3, kind 0 or 1). */
 int sp_tuned_config(sp_convection* h, int precision, int batch, int op, int* ty, int* zchunk, int* kind);
 /* Runs the autotuner for this handle's grid at `batch` fields and precision: every
- * stage kernel gets the fastest of its candidate launch shapes, and FP64 RK4
+ * stage kernel gets the fastest of its candidate launch shapes (whole steps decide
+ * between those, a chain of direct kernels and what an untuned handle runs), and FP64 RK4
  * steps run as fused pairs when those are more than 2 % faster than the four
  * stages: for batch 1 as timed through sp_do_rk4 (a graph chunk of 50 steps on
  * scratch fields), for larger batches over four consecutive batched steps, each
@@ -288,7 +292,7 @@ int sp_tuned_config(sp_convection* h, int precision, int batch, int op, int* ty,
  * on their best 32 x 16 tiles, which are kept unless more than 1 % slower
  * (they move fewer DRAM bytes, so they hold a higher clock under the cap).
  * Small FP64 fields then take a cluster-resident path (kind 3 or 5 of
- * sp_set_tune) when it is faster.  Takes about 1-3 s. */
+ * sp_set_tune) when it is faster than the best of those, over 50 steps.  Takes about 1-3 s. */
 int sp_autotune(sp_convection* h, int precision, int batch);
 /* Test of the error path of the bounded in-kernel waits: runs one kernel whose
  * wait can never complete and gives up after limit_ms (<= 2000); returns

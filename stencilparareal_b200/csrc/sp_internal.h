@@ -144,7 +144,8 @@ Shape default_stage_shape(const Geo& g, int items, bool adjoint = false);
 bool wrap_supported(const Geo& g);
 
 // Items with a diffusivity of their own that one launch takes (their weights are
-// kernel arguments, 104 bytes each: within 4 KB); larger batches take several.
+// kernel arguments, 104 bytes each: 4.1 KB with the four tensor maps of a TMA stage);
+// larger batches take several.
 constexpr int kItemWeights = 32;
 
 // The stage, pair and cluster kernels access fields in 16-byte chunks: their launches

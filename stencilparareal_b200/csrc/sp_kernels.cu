@@ -279,7 +279,7 @@ __device__ __forceinline__ void reduce_par(double* g, double* par_acc, double gs
 // Bound by latency at the sizes it is for: below ~4M FP64 cells a stage is one
 // short wave, and what counts is the time from launch to the last store.  Hence
 // no barrier and no shared-memory ring to fill, few registers (50-64 for the
-// FP64 RK stages: 16 or more blocks of 128 threads per SM), a compact plane loop
+// FP64 RK stages: 8 to 10 blocks of 128 threads per SM), a compact plane loop
 // (not unrolled: 2-3 KB of code per stage instead of 10-25 KB, which the short
 // kernels spent their time fetching) and programmatic dependent launch.  us per
 // RK4 step, one-thread-per-cell direct kernel / best TMA ring / this kernel:
@@ -814,7 +814,7 @@ cudaError_t launch_direct_T(const Geo& g, const StageLaunch& L, KArgs<T> a, cons
     fill_weights(wt, L.coef, L.nu, L.nu_items, L.items);
     auto run = [&](auto k) { return launch_in_stream(!L.drain, k, grid, dim3(threads), 0, s, a, wt); };
     if (L.wrap) {
-        constexpr int ZMAX = OpTraits<OP>::adjoint ? 2 : 4;  // (adjoint stages: 100 registers with two planes)
+        constexpr int ZMAX = OpTraits<OP>::adjoint ? 2 : 4;  // (adjoint stages: 80-86 registers)
         switch (std::min(t.zchunk, ZMAX)) {
             case 1: return run(k_stage_wrap<T, OP, NW, 1>);
             case 2: return run(k_stage_wrap<T, OP, NW, 2>);
