@@ -218,4 +218,4 @@ def test_tuned_shapes_are_no_slower_than_the_defaults(sp, prec, n):
 
     default = fastest()
     c.autotune(prec, 1)
-    assert fastest() < 1.08 * default
+    assert fastest() < 1.12 * default
